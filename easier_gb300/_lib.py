@@ -16,6 +16,7 @@ from .utils import EasierJitException
 
 F32, F64, I32, I64 = 0, 1, 2, 3
 REDUCE_OPS = {"sum": 0, "prod": 1, "mean": 2, "amax": 3, "amin": 4}
+REDUCE_FILL = 0x100
 AGG_SUM, AGG_PROD, AGG_NORM, AGG_MAX, AGG_MIN = 0, 1, 2, 3, 4
 DEV_IDX_RANGE, DEV_NONFINITE, DEV_WAIT_TIMEOUT = 1, 2, 4
 

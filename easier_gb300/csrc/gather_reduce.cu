@@ -1,9 +1,9 @@
 // Selector gather, Reducer segmented reduce, aggregators and dot products.
 //
 // Everything here is deterministic: there are no floating-point atomics.
-// Segmented reductions run one thread per (row, column) and walk the segment
-// in ascending order, which is the order the reference's CPU
-// scatter_reduce_ accumulates in, so sums are bitwise equal to it.
+// Segmented reductions run one thread per row and walk the segment in
+// ascending order, which is the order the reference's CPU scatter_reduce_
+// accumulates in, so sums are bitwise equal to it.
 #include <cmath>
 #include <cstdint>
 #include <mutex>
@@ -15,116 +15,380 @@ namespace {
 
 constexpr int kThreads = 256;
 
-int grid_for(int64_t work, int threads = kThreads) {
-  int64_t g = (work + threads - 1) / threads;
-  if (g < 1) g = 1;
-  if (g > 152 * 32) g = 152 * 32;  // grid-stride beyond 32 CTAs per SM
-  return (int)g;
+// Local element -> (row, column) of a tile without a division: j / d for
+// j < 2^16 and 1 <= d < 2^16 is umulhi(j, ceil(2^32 / d)) exactly (the
+// rounding error of the quotient, j * (d - 1) / (d * 2^32), stays below 1/d).
+struct FastDiv {
+  uint32_t d, magic;
+};
+
+inline FastDiv fast_div(uint32_t d) { return FastDiv{d, d > 1 ? (uint32_t)((((uint64_t)1 << 32) + d - 1) / d) : 0u}; }
+
+template <int D>
+__device__ __forceinline__ uint32_t div_by(uint32_t j, FastDiv f) {
+  if (D > 0) return j / (uint32_t)(D > 0 ? D : 1);
+  return f.d > 1 ? __umulhi(j, f.magic) : j;
 }
 
 // ---------------------------------------------------------------- gather --
-template <typename V>
+// Bound: HBM, given enough loads in flight (index -> row is a chain of two
+// dependent loads) and few enough instructions a vector.  A CTA takes a tile
+// of whole rows (or of up to kGatherCols vectors of long rows, blockIdx.y) of
+// about U * kThreads vectors; a thread requests U indices, then U row
+// vectors, strided so that every store and index load is coalesced.  In a
+// tile of whole rows vector j goes to offset j, and its (row, column) is a
+// 16-bit division (FastDiv).  A 64-bit division per vector and one load in
+// flight a thread, as before, took 59 us for 5.87 M rows of 12 bytes (this
+// form 37, whole rows a thread as below 25: 4.7 TB/s of the bytes it must
+// move).
+constexpr int kGatherCols = 1024;  // vectors of one row a tile takes at most
+
+// O: type of a vector's offset in x (32 bits where x is small enough)
+template <typename V, int D, int U, typename O>
 __global__ void __launch_bounds__(kThreads)
-gather_kernel(const V *__restrict__ x, int64_t n_in, int64_t vpr,
-              const int32_t *__restrict__ idx, int64_t m, V *__restrict__ y) {
-  const int64_t total = m * vpr;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += stride) {
-    int64_t e, c;
-    if (vpr == 1) {
-      e = t;
-      c = 0;
-    } else {
-      e = t / vpr;
-      c = t - e * vpr;
+gather_kernel(const V *__restrict__ x, uint32_t n_in, O vpr, const int32_t *__restrict__ idx, int64_t m,
+              V *__restrict__ y, int rows_per_tile, FastDiv cols, int64_t col0) {
+  const int64_t row0 = (int64_t)blockIdx.x * rows_per_tile;
+  const O c0 = D > 0 ? O(0) : (O)(col0 + (int64_t)blockIdx.y * kGatherCols);
+  const uint32_t rows = (uint32_t)(m - row0 < rows_per_tile ? m - row0 : rows_per_tile);
+  const uint32_t width = D > 0 ? (uint32_t)D : (uint32_t)((int64_t)vpr - (int64_t)c0 < cols.d ? (int64_t)vpr - (int64_t)c0 : cols.d);
+  const O row_len = D > 0 ? (O)D : vpr;
+  const uint32_t count = rows * width;  // (a row cut into column blocks: one row a tile, no division)
+  const bool cut = D == 0 && (int64_t)vpr > kGatherCols;
+  const int32_t *__restrict__ ti = idx + row0;
+  V *__restrict__ ty = y + row0 * (int64_t)row_len + (int64_t)c0;
+  for (uint32_t j0 = threadIdx.x; j0 < count; j0 += U * kThreads) {
+    uint32_t s[U], c[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint32_t j = j0 + u * kThreads;
+      const uint32_t r = cut ? 0u : div_by<D>(j, cols);
+      c[u] = j - r * width;
+      s[u] = j < count ? (uint32_t)__ldg(ti + r) : 0u;
     }
-    const int32_t s = __ldg(idx + e);
-    if (s < 0 || (int64_t)s >= n_in) {
-      esr::raise_status(ESR_DEV_IDX_RANGE);
-      continue;
+    V v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (s[u] < n_in) v[u] = x[(O)s[u] * row_len + c0 + c[u]];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint32_t j = j0 + u * kThreads;
+      if (j < count) {
+        if (s[u] < n_in) ty[j] = v[u];
+        else esr::raise_status(ESR_DEV_IDX_RANGE);
+      }
     }
-    y[t] = x[(int64_t)s * vpr + c];
+  }
+}
+
+// Rows of D (3) vectors: a thread takes U whole rows, whose vectors go through
+// shared memory to coalesced stores.  A third of the index work of the kernel
+// above: 28 -> 25 us for 5.87 M rows of three floats.
+template <typename V, int D, int U, typename O>
+__global__ void __launch_bounds__(kThreads)
+gather_rows_kernel(const V *__restrict__ x, uint32_t n_in, const int32_t *__restrict__ idx, int64_t m,
+                   V *__restrict__ y) {
+  __shared__ V s_row[kThreads * D];
+  __shared__ uint8_t s_ok[kThreads];
+  const int64_t row0 = (int64_t)blockIdx.x * (U * kThreads);
+  uint32_t s[U];
+  V v[U][D];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const int64_t e = row0 + u * kThreads + threadIdx.x;
+    s[u] = e < m ? (uint32_t)__ldg(idx + e) : 0u;
+  }
+#pragma unroll
+  for (int u = 0; u < U; ++u)
+#pragma unroll
+    for (int c = 0; c < D; ++c)
+      if (s[u] < n_in) v[u][c] = x[(O)s[u] * D + c];
+  V *const warp_rows = s_row + (threadIdx.x & ~31) * D;
+  uint8_t *const warp_ok = s_ok + (threadIdx.x & ~31);
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int u = 0; u < U; ++u) {  // each warp stages its own 32 rows
+    const int64_t e0 = row0 + u * kThreads + (threadIdx.x & ~31);
+    const bool here = e0 + lane < m, ok = here && s[u] < n_in;
+    if (here && !ok) esr::raise_status(ESR_DEV_IDX_RANGE);
+    __syncwarp();
+    if (ok) {
+#pragma unroll
+      for (int c = 0; c < D; ++c) warp_rows[lane * D + c] = v[u][c];
+    }
+    warp_ok[lane] = ok;
+    __syncwarp();
+#pragma unroll
+    for (int c = 0; c < D; ++c) {
+      const int j = lane + 32 * c;
+      if (warp_ok[j / D]) y[e0 * D + j] = warp_rows[j];
+    }
+  }
+}
+
+template <typename V, int D, int U>
+void launch_gather_rows(const V *x, int64_t n_in, const int32_t *idx, int64_t m, V *y, cudaStream_t st) {
+  const unsigned g = (unsigned)((m + U * kThreads - 1) / (U * kThreads));
+  const uint32_t nin = n_in > ((int64_t)1 << 31) ? (uint32_t)1 << 31 : (uint32_t)n_in;
+  if (n_in * D < ((int64_t)1 << 31)) gather_rows_kernel<V, D, U, uint32_t><<<g, kThreads, 0, st>>>(x, nin, idx, m, y);
+  else gather_rows_kernel<V, D, U, int64_t><<<g, kThreads, 0, st>>>(x, nin, idx, m, y);
+}
+
+template <typename V, int D, int U>
+void launch_gather_u(const V *x, int64_t n_in, int64_t vpr, const int32_t *idx, int64_t m, V *y, cudaStream_t st) {
+  const int width = (int)(vpr < kGatherCols ? vpr : kGatherCols);
+  const int rows = width >= U * kThreads ? 1 : U * kThreads / width;
+  const int64_t gx = (m + rows - 1) / rows;
+  // indices are int32: none of them reaches 2^31
+  const uint32_t nin = n_in > ((int64_t)1 << 31) ? (uint32_t)1 << 31 : (uint32_t)n_in;
+  for (int64_t c0 = 0; c0 < vpr; c0 += (int64_t)65535 * kGatherCols) {
+    int64_t gy = (vpr - c0 + kGatherCols - 1) / kGatherCols;
+    if (gy > 65535) gy = 65535;
+    const dim3 g((unsigned)gx, (unsigned)gy);
+    if (n_in * vpr < ((int64_t)1 << 31))
+      gather_kernel<V, D, U, uint32_t><<<g, kThreads, 0, st>>>(x, nin, (uint32_t)vpr, idx, m, y, rows, fast_div(width), c0);
+    else
+      gather_kernel<V, D, U, int64_t><<<g, kThreads, 0, st>>>(x, nin, vpr, idx, m, y, rows, fast_div(width), c0);
   }
 }
 
 template <typename V>
-int launch_gather(const void *x, int64_t n_in, int64_t row_bytes, const int32_t *idx, int64_t m,
-                  void *y, cudaStream_t st) {
+int launch_gather(const void *x, int64_t n_in, int64_t row_bytes, const int32_t *idx, int64_t m, void *y,
+                  cudaStream_t st) {
   const int64_t vpr = row_bytes / (int64_t)sizeof(V);
-  gather_kernel<V><<<grid_for(m * vpr), kThreads, 0, st>>>((const V *)x, n_in, vpr, idx, m, (V *)y);
+  const V *xv = (const V *)x;
+  V *yv = (V *)y;
+  // four vectors a thread once that still gives every SM eight CTAs
+  const bool wide = m * vpr >= (int64_t)152 * 8 * 4 * kThreads;
+  if (vpr == 1) {
+    if (wide) launch_gather_u<V, 1, 4>(xv, n_in, vpr, idx, m, yv, st);
+    else launch_gather_u<V, 1, 1>(xv, n_in, vpr, idx, m, yv, st);
+  } else if (vpr == 3) {
+    if (wide) launch_gather_rows<V, 3, 2>(xv, n_in, idx, m, yv, st);
+    else launch_gather_rows<V, 3, 1>(xv, n_in, idx, m, yv, st);
+  } else {
+    if (wide) launch_gather_u<V, 0, 4>(xv, n_in, vpr, idx, m, yv, st);
+    else launch_gather_u<V, 0, 1>(xv, n_in, vpr, idx, m, yv, st);
+  }
   ESR_LAUNCH_CHECK("esr_gather");
   return ESR_OK;
 }
 
 // ----------------------------------------------------------- segreduce --
 template <typename T>
-struct Acc {  // accumulation type
-  using type = T;
-};
-
-template <typename T>
 __device__ __forceinline__ bool is_nan(T v) {
   return v != v;
 }
 
+// 0 + v without an add (the FP64 pipe is GB300's scarce one): v, with -0
+// turned into +0
+__device__ __forceinline__ double plus_zero(double v) {
+  return __double_as_longlong(v) == (long long)0x8000000000000000ull ? 0.0 : v;
+}
+__device__ __forceinline__ float plus_zero(float v) { return __fadd_rn(0.f, v); }
+__device__ __forceinline__ int32_t plus_zero(int32_t v) { return v; }
+__device__ __forceinline__ int64_t plus_zero(int64_t v) { return v; }
+
 template <typename T, int OP>
-__global__ void __launch_bounds__(kThreads)
-segreduce_kernel(const T *__restrict__ t, int64_t cols, const int32_t *__restrict__ rowptr,
-                 const int32_t *__restrict__ perm, int64_t n, T *__restrict__ out) {
-  const int64_t total = n * cols;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g < total; g += stride) {
-    int64_t i, c;
-    if (cols == 1) {
-      i = g;
-      c = 0;
-    } else {
-      i = g / cols;
-      c = g - i * cols;
-    }
-    const int32_t b = __ldg(rowptr + i), e = __ldg(rowptr + i + 1);
-    if (b >= e) continue;  // unreferenced row keeps `out`
-    T acc;
-    if (OP == ESR_REDUCE_SUM || OP == ESR_REDUCE_MEAN) acc = T(0);
-    else if (OP == ESR_REDUCE_PROD) acc = T(1);
-    for (int32_t k = b; k < e; ++k) {
-      const int64_t src = perm ? (int64_t)__ldg(perm + k) : (int64_t)k;
-      const T v = t[src * cols + c];
-      if (OP == ESR_REDUCE_SUM || OP == ESR_REDUCE_MEAN) acc = ops<T>::add(acc, v);
-      else if (OP == ESR_REDUCE_PROD) acc = ops<T>::mul(acc, v);
-      else if (OP == ESR_REDUCE_AMAX) {
-        if (k == b) acc = v;
-        else acc = is_nan(v) ? v : ((acc < v) ? v : acc);
-      } else {
-        if (k == b) acc = v;
-        else acc = is_nan(v) ? v : ((v < acc) ? v : acc);
+__device__ __forceinline__ T seg_combine(T acc, T v, bool first) {
+  if (OP == ESR_REDUCE_SUM || OP == ESR_REDUCE_MEAN) return first ? plus_zero(v) : ops<T>::add(acc, v);
+  if (OP == ESR_REDUCE_PROD) return first ? v : ops<T>::mul(acc, v);
+  if (first || is_nan(v)) return v;
+  if (OP == ESR_REDUCE_AMAX) return (acc < v) ? v : acc;
+  return (v < acc) ? v : acc;
+}
+
+// The largest of the warp's values (a warp-uniform trip count: FP64
+// instructions that are predicated off for every lane still take their pipe).
+__device__ __forceinline__ int32_t warp_most(int32_t v) { return __reduce_max_sync(0xffffffffu, v); }
+
+// One thread per row (of D columns, or of one of them), its entries in
+// ascending order.  Bound: HBM, given enough loads in flight: a row is a chain
+// row bounds -> perm -> value, so a thread requests R rows' bounds, then up to
+// U positions of each, then their values, before it adds them in order;
+// longer segments go on U entries at a time.  Load::entry(k) gives an entry's
+// position, fetch() loads what lies there, value() turns that into the terms.
+// Rows without entries reach the store with `none` set.  (Staging the entries
+// through shared memory so that perm loads coalesce was slower: 131 us against
+// 52 for a plain loop per (row, column) at 1.96 M rows of 3 entries x 3 FP32
+// columns; a thread per row takes 24, 5.2 TB/s.)
+// Every thread of the warp calls it.
+template <typename T, int OP, int D, int U, int R, class Load, class Store>
+__device__ __forceinline__ void seg_rows(const Load &load, const Store &store, const int32_t *__restrict__ rowptr,
+                                         const int64_t (&row)[R], const int64_t (&col)[R], const bool (&mine)[R]) {
+  int32_t b[R], e[R];
+#pragma unroll
+  for (int q = 0; q < R; ++q) {
+    b[q] = mine[q] ? __ldg(rowptr + row[q]) : 0;
+    e[q] = mine[q] ? __ldg(rowptr + row[q] + 1) : 0;
+  }
+  typename Load::Held h[R][U];
+  int32_t src[R][U];
+#pragma unroll
+  for (int q = 0; q < R; ++q)
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (u < e[q] - b[q]) src[q][u] = load.entry(b[q] + u);
+#pragma unroll
+  for (int q = 0; q < R; ++q)
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (u < e[q] - b[q]) load.fetch(src[q][u], col[q], h[q][u]);
+#pragma unroll
+  for (int q = 0; q < R; ++q) {
+    T acc[D];
+#pragma unroll
+    for (int c = 0; c < D; ++c) acc[c] = T(0);
+    const int32_t most = warp_most(e[q] - b[q]);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (u >= most) break;
+      if (u < e[q] - b[q]) {
+        T v[D];
+        load.value(h[q][u], v);
+#pragma unroll
+        for (int c = 0; c < D; ++c) acc[c] = seg_combine<T, OP>(acc[c], v[c], u == 0);
       }
     }
-    if (OP == ESR_REDUCE_MEAN) acc = ops<T>::div_count(acc, (int64_t)(e - b));
-    out[i * cols + c] = acc;
+    for (int32_t done = U; done < most; done += U) {
+      const int32_t left = e[q] - b[q] - done;
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (u < left) src[q][u] = load.entry(b[q] + done + u);
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (u < left) load.fetch(src[q][u], col[q], h[q][u]);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (u >= most - done) break;
+        if (u < left) {
+          T v[D];
+          load.value(h[q][u], v);
+#pragma unroll
+          for (int c = 0; c < D; ++c) acc[c] = seg_combine<T, OP>(acc[c], v[c], false);
+        }
+      }
+    }
+    if (!mine[q]) continue;
+    if (OP == ESR_REDUCE_MEAN && b[q] < e[q]) {
+#pragma unroll
+      for (int c = 0; c < D; ++c) acc[c] = ops<T>::div_count(acc[c], (int64_t)(e[q] - b[q]));
+    }
+    store(row[q], col[q], acc, b[q] >= e[q]);
+  }
+}
+
+// t[perm[k], c .. c + D)
+template <typename T, int D>
+struct SegLoad {
+  struct Held {
+    T v[D];
+  };
+  const T *t;
+  int64_t cols;
+  const int32_t *perm;
+  __device__ __forceinline__ int32_t entry(int32_t k) const { return perm ? __ldg(perm + k) : k; }
+  __device__ __forceinline__ void fetch(int32_t src, int64_t c0, Held &h) const {
+    const T *p = t + ((int64_t)src * (D > 1 ? (int64_t)D : cols) + c0);
+#pragma unroll
+    for (int c = 0; c < D; ++c) h.v[c] = __ldg(p + c);
+  }
+  __device__ __forceinline__ void value(const Held &h, T (&v)[D]) const {
+#pragma unroll
+    for (int c = 0; c < D; ++c) v[c] = h.v[c];
+  }
+};
+
+template <typename T, int D>
+struct SegStore {
+  T *out;
+  int64_t cols;
+  bool fill;  // rows without entries get zero (otherwise they keep `out`)
+  __device__ __forceinline__ void operator()(int64_t i, int64_t c0, const T (&acc)[D], bool none) const {
+    T *p = out + (i * (D > 1 ? (int64_t)D : cols) + c0);
+    if (!none || fill) {
+#pragma unroll
+      for (int c = 0; c < D; ++c) p[c] = acc[c];
+    }
+  }
+};
+
+// Narrow rows (1..4 columns): a thread takes R whole rows, kThreads apart.
+template <typename T, int OP, int D, int R>
+__global__ void __launch_bounds__(kThreads)
+segreduce_kernel(const T *__restrict__ t, const int32_t *__restrict__ rowptr, const int32_t *__restrict__ perm,
+                 int64_t n, T *__restrict__ out, int fill) {
+  int64_t row[R], col[R];
+  bool mine[R];
+#pragma unroll
+  for (int q = 0; q < R; ++q) {
+    row[q] = ((int64_t)blockIdx.x * R + q) * kThreads + threadIdx.x;
+    col[q] = 0;
+    mine[q] = row[q] < n;
+  }
+  seg_rows<T, OP, D, 4, R>(SegLoad<T, D>{t, 1, perm}, SegStore<T, D>{out, 1, fill != 0}, rowptr, row, col, mine);
+}
+
+// Wider rows: a CTA takes `rows` consecutive rows times up to kThreads columns
+// (blockIdx.y), a thread one (row, column).
+template <typename T, int OP>
+__global__ void __launch_bounds__(kThreads)
+segreduce_cols_kernel(const T *__restrict__ t, int64_t cols, const int32_t *__restrict__ rowptr,
+                      const int32_t *__restrict__ perm, int64_t n, T *__restrict__ out, int rows, FastDiv width,
+                      int64_t col0, int fill) {
+  const int64_t row0 = (int64_t)blockIdx.x * rows;
+  const int64_t c0 = col0 + (int64_t)blockIdx.y * kThreads;
+  const uint32_t w = (uint32_t)(cols - c0 < width.d ? cols - c0 : width.d);
+  const uint32_t r = cols > kThreads ? 0u : div_by<0>(threadIdx.x, width), c = threadIdx.x - r * w;
+  const int64_t row[1] = {row0 + r}, col[1] = {c0 + c};
+  const bool mine[1] = {r < (uint32_t)rows && row0 + r < n && c < w};
+  seg_rows<T, OP, 1, 4, 1>(SegLoad<T, 1>{t, cols, perm}, SegStore<T, 1>{out, cols, fill != 0}, rowptr, row, col, mine);
+}
+
+template <typename T, int OP, int D>
+void launch_seg_rows(const T *t, const int32_t *rowptr, const int32_t *perm, int64_t n, T *out, int fill,
+                     cudaStream_t st) {
+  // two rows a thread once that still gives every SM eight CTAs
+  if (n >= (int64_t)152 * 8 * 2 * kThreads)
+    segreduce_kernel<T, OP, D, 2><<<(unsigned)((n + 2 * kThreads - 1) / (2 * kThreads)), kThreads, 0, st>>>(
+        t, rowptr, perm, n, out, fill);
+  else
+    segreduce_kernel<T, OP, D, 1><<<(unsigned)((n + kThreads - 1) / kThreads), kThreads, 0, st>>>(t, rowptr, perm, n,
+                                                                                                  out, fill);
+}
+
+template <typename T, int OP>
+void launch_seg_op(const T *t, int64_t cols, const int32_t *rowptr, const int32_t *perm, int64_t n, T *out, int fill,
+                   cudaStream_t st) {
+  switch (cols) {
+    case 1: return launch_seg_rows<T, OP, 1>(t, rowptr, perm, n, out, fill, st);
+    case 2: return launch_seg_rows<T, OP, 2>(t, rowptr, perm, n, out, fill, st);
+    case 3: return launch_seg_rows<T, OP, 3>(t, rowptr, perm, n, out, fill, st);
+    case 4: return launch_seg_rows<T, OP, 4>(t, rowptr, perm, n, out, fill, st);
+    default: break;
+  }
+  const int width = (int)(cols < kThreads ? cols : kThreads);
+  const int rows = kThreads / width;
+  for (int64_t c0 = 0; c0 < cols; c0 += (int64_t)65535 * kThreads) {
+    int64_t gy = (cols - c0 + kThreads - 1) / kThreads;
+    if (gy > 65535) gy = 65535;
+    segreduce_cols_kernel<T, OP><<<dim3((unsigned)((n + rows - 1) / rows), (unsigned)gy), kThreads, 0, st>>>(
+        t, cols, rowptr, perm, n, out, rows, fast_div(width), c0, fill);
   }
 }
 
 template <typename T>
 int launch_segreduce(int op, const void *t, int64_t cols, const int32_t *rowptr, const int32_t *perm,
                      int64_t n, void *out, cudaStream_t st) {
-  const int g = grid_for(n * cols);
-  switch (op) {
-    case ESR_REDUCE_SUM:
-      segreduce_kernel<T, ESR_REDUCE_SUM><<<g, kThreads, 0, st>>>((const T *)t, cols, rowptr, perm, n, (T *)out);
-      break;
-    case ESR_REDUCE_PROD:
-      segreduce_kernel<T, ESR_REDUCE_PROD><<<g, kThreads, 0, st>>>((const T *)t, cols, rowptr, perm, n, (T *)out);
-      break;
-    case ESR_REDUCE_MEAN:
-      segreduce_kernel<T, ESR_REDUCE_MEAN><<<g, kThreads, 0, st>>>((const T *)t, cols, rowptr, perm, n, (T *)out);
-      break;
-    case ESR_REDUCE_AMAX:
-      segreduce_kernel<T, ESR_REDUCE_AMAX><<<g, kThreads, 0, st>>>((const T *)t, cols, rowptr, perm, n, (T *)out);
-      break;
-    case ESR_REDUCE_AMIN:
-      segreduce_kernel<T, ESR_REDUCE_AMIN><<<g, kThreads, 0, st>>>((const T *)t, cols, rowptr, perm, n, (T *)out);
-      break;
+  const int fill = (op & ESR_REDUCE_FILL) ? 1 : 0;
+  const T *tv = (const T *)t;
+  T *ov = (T *)out;
+  switch (op & ~ESR_REDUCE_FILL) {
+    case ESR_REDUCE_SUM: launch_seg_op<T, ESR_REDUCE_SUM>(tv, cols, rowptr, perm, n, ov, fill, st); break;
+    case ESR_REDUCE_PROD: launch_seg_op<T, ESR_REDUCE_PROD>(tv, cols, rowptr, perm, n, ov, fill, st); break;
+    case ESR_REDUCE_MEAN: launch_seg_op<T, ESR_REDUCE_MEAN>(tv, cols, rowptr, perm, n, ov, fill, st); break;
+    case ESR_REDUCE_AMAX: launch_seg_op<T, ESR_REDUCE_AMAX>(tv, cols, rowptr, perm, n, ov, fill, st); break;
+    case ESR_REDUCE_AMIN: launch_seg_op<T, ESR_REDUCE_AMIN>(tv, cols, rowptr, perm, n, ov, fill, st); break;
     default:
       return esr::fail(ESR_ERR_ARG, "unknown reduce op");
   }

@@ -113,6 +113,7 @@ def _load_reducer(red: _m.Reducer, device) -> None:
         red.idx = torch.from_numpy(idx_np).to(device)
         red._rowptr32 = torch.from_numpy(rowptr.astype(np.int32)).to(device)
         red._perm32 = torch.from_numpy(perm.astype(np.int32)).to(device)
+    red._in_row_order = bool((idx[1:] >= idx[:-1]).all())
     red.easier_index_status = "rewritten"
     red.set_is_full()
 

@@ -163,6 +163,7 @@ class Reducer(nn.Module):
         # original element order) as int32 device tensors
         self._rowptr32: Optional[torch.Tensor] = None
         self._perm32: Optional[torch.Tensor] = None
+        self._in_row_order: bool = False  # idx ascending: the permutation is the identity
         self.easier_is_full: bool = False
 
     def set_is_full(self):
@@ -173,10 +174,7 @@ class Reducer(nn.Module):
     def forward(self, tensor: torch.Tensor, *, out: Optional[torch.Tensor] = None) -> torch.Tensor:
         if self.easier_index_status != "rewritten":
             raise RuntimeError("Reducer.idx not ready, run compile() first")
-        shape = tensor.shape
-        if out is None:
-            out = torch.zeros((self.n,) + tuple(shape[1:]), dtype=tensor.dtype, device=tensor.device)
-        if out.shape[0] != self.n:
+        if out is not None and out.shape[0] != self.n:
             raise ValueError(
                 f"{out.shape[0]} the length of the first dimension of `out`"
                 f" and {self.n} the specified `Reducer.n` do not match")

@@ -6,6 +6,8 @@ current stream.  Non-CUDA tensors raise: there is no CPU path.
 """
 from __future__ import annotations
 
+from typing import Optional
+
 import torch
 
 from . import _lib
@@ -34,12 +36,24 @@ def select(sel, tensor: torch.Tensor) -> torch.Tensor:
     return out
 
 
-def reduce(red, tensor: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
+def _perm_ptr(red):
+    """The Reducer's permutation, or NULL where it is the identity (edges
+    already in row order: the kernels then need not read it)."""
+    return None if red._in_row_order else _lib.ptr(red._perm32)
+
+
+def reduce(red, tensor: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Reducer.forward: out.scatter_reduce_(0, idx, t, op, include_self=False)
     (easier/core/module.py:441-461), as a deterministic in-order segment
-    reduction over the CSR of idx."""
+    reduction over the CSR of idx.  Without ``out`` the kernel writes the
+    zeros of unreferenced rows itself."""
     _require_cuda(tensor, "Reducer")
-    _require_cuda(out, "Reducer out")
+    op = _lib.REDUCE_OPS[red.reduce]
+    if out is None:
+        out = torch.empty((red.n,) + tuple(tensor.shape[1:]), dtype=tensor.dtype, device=tensor.device)
+        op |= _lib.REDUCE_FILL
+    else:
+        _require_cuda(out, "Reducer out")
     if tensor.dtype != out.dtype:
         raise RuntimeError(f"scatter_reduce(): Expected self.dtype to be equal to src.dtype ({out.dtype} vs {tensor.dtype})")
     m = red._perm32.shape[0]
@@ -50,8 +64,8 @@ def reduce(red, tensor: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
     src = tensor.contiguous()
     dst = out if out.is_contiguous() else out.contiguous()
     cols = int(torch.Size(src.shape[1:]).numel())
-    _lib.call("esr_segreduce", _lib.dtype_code(src.dtype), _lib.REDUCE_OPS[red.reduce], _lib.ptr(src), cols,
-              _lib.ptr(red._rowptr32), _lib.ptr(red._perm32), red.n, _lib.ptr(dst), _lib.stream_handle(src.device))
+    _lib.call("esr_segreduce", _lib.dtype_code(src.dtype), op, _lib.ptr(src), cols, _lib.ptr(red._rowptr32),
+              _perm_ptr(red), red.n, _lib.ptr(dst), _lib.stream_handle(src.device))
     if dst is not out:
         out.copy_(dst)
     return out

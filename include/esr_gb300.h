@@ -44,6 +44,9 @@ enum {
   ESR_REDUCE_AMAX = 3,
   ESR_REDUCE_AMIN = 4
 };
+/* added to the op of esr_segreduce: rows with an empty segment get zero
+ * (Reducer.forward without `out`: module.py:448-450) */
+#define ESR_REDUCE_FILL 0x100
 
 /* aggregators: easier/core/module.py:825-884 (sum, prod, norm, max, min) */
 enum {
@@ -202,7 +205,8 @@ int esr_gather(const void *x, int64_t n_in, int64_t row_bytes,
 /* Deterministic segmented reduce over a CSR segmentation:
  *   out[i, c] = op over k in [rowptr[i], rowptr[i+1]) of t[perm ? perm[k] : k, c]
  * in ascending k (the reference's in-segment edge order).  Rows with an empty
- * segment keep `out` unchanged (scatter_reduce_ with include_self=False).
+ * segment keep `out` unchanged (scatter_reduce_ with include_self=False), or
+ * get zero with op | ESR_REDUCE_FILL.
  * Replaces easier/core/module.py:441-461 (Reducer.forward).
  * dtype: ESR_F32/F64/I32/I64; op: ESR_REDUCE_*. */
 int esr_segreduce(int dtype, int op, const void *t, int64_t row_elems,

@@ -1,0 +1,81 @@
+"""Selector, Reducer, Linsys and aggregator kernels at the sizes where their
+tiling can go wrong: tile edges, remainders, long segments, wide rows, every
+dispatch branch.  Bitwise against the oracle (order-fixed work) or the
+op-by-op path; sums within the rounding bound n * 2^-53 * sum |x|."""
+import numpy as np
+import pytest
+import torch
+
+import easier_gb300 as esr
+from oracle import sparse as osp
+
+pytestmark = pytest.mark.gpu
+
+
+def _module(sel=None, red=None, n=0, op="sum"):
+    class M(esr.Module):
+        def __init__(self):
+            super().__init__()
+            if sel is not None:
+                self.sel = esr.Selector(sel)
+            if red is not None:
+                self.red = esr.Reducer(red, n, op)
+    m = M()
+    esr.compile([m], "cuda")
+    return m
+
+
+@pytest.mark.parametrize("m", [1, 255, 257, 1025, 1_300_000])
+@pytest.mark.parametrize("dtype,tail", [(torch.uint8, (3,)), (torch.float32, ()), (torch.float32, (3,)),
+                                        (torch.float64, (3,)), (torch.float32, (4,)), (torch.int64, (7,))])
+def test_gather_tiles(m, dtype, tail):
+    g = torch.Generator().manual_seed(m)
+    n = 1000
+    idx = torch.randint(0, n, (m,), generator=g)
+    x = torch.randint(0, 200, (n,) + tail, generator=g).to(dtype)
+    assert torch.equal(_module(sel=idx).sel(x.cuda()).cpu(), x[idx])
+
+
+@pytest.mark.parametrize("cols", [1023, 1024, 1025, 4100])
+def test_gather_wide_rows(cols):
+    g = torch.Generator().manual_seed(cols)
+    idx = torch.randint(0, 37, (50,), generator=g)
+    x = torch.randn(37, cols, generator=g)
+    mod = _module(sel=idx)
+    assert torch.equal(mod.sel(x.cuda()).cpu(), x[idx])
+    y = torch.randn(37, cols + 1, generator=g)[:, 1:].contiguous()  # odd 4-byte offsets
+    flat = torch.cat([torch.zeros(1), y.reshape(-1)]).cuda()[1:].view(37, cols)
+    assert torch.equal(mod.sel(flat).cpu(), y[idx])
+
+
+@pytest.mark.parametrize("op", ["sum", "mean", "prod", "amax", "amin"])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64, torch.int64])
+@pytest.mark.parametrize("cols", [1, 2, 3, 5, 255, 256, 257])
+def test_segments(op, dtype, cols):
+    """Rows without entries, rows longer than a staged chunk, a last tile cut
+    short; sorted indices (no permutation) and shuffled ones."""
+    if op in ("mean", "prod") and not dtype.is_floating_point:
+        pytest.skip("floating reductions")
+    g = torch.Generator().manual_seed(cols)
+    n = 301 if cols < 100 else 7
+    long = torch.full((2500,), 2) if cols < 100 else torch.full((40,), 2)
+    idx = torch.cat([torch.randint(0, n - 2, (900 if cols < 100 else 60,), generator=g), long])
+    idx[idx == 4] = 5  # row 4 and the last row stay empty
+    for shuffled in (False, True):
+        i = idx[torch.randperm(idx.shape[0], generator=g)] if shuffled else idx.sort().values
+        t = torch.randn(i.shape[0], *(() if cols == 1 else (cols,)), generator=g, dtype=torch.float64)
+        t = (t if dtype.is_floating_point else t * 1000).to(dtype)
+        if dtype.is_floating_point:
+            t[3] = -0.0
+            if op.startswith("a"):
+                t[7] = float("nan")
+                t[9] = float("inf")
+        mod = _module(red=i, n=n, op=op)
+        assert mod.red._in_row_order == (not shuffled)
+        got, want = mod.red(t.cuda()).cpu(), osp.reduce(t, i, n, op)
+        assert np.array_equal(got.numpy(), want.numpy(), equal_nan=dtype.is_floating_point)
+        out = torch.full_like(want, 3)
+        kept = mod.red(t.cuda(), out=out.cuda()).cpu()
+        empty = torch.bincount(i, minlength=n) == 0
+        assert torch.equal(kept[empty], out[empty]) and int(empty.sum()) >= 2
+        assert np.array_equal(kept[~empty].numpy(), want[~empty].numpy(), equal_nan=dtype.is_floating_point)
