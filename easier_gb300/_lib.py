@@ -104,6 +104,7 @@ _SIGS = {
     "esr_sell_build": (c_int, [c_int64, _P, _P, _P, c_int64, _P, _P, _P]),
     "esr_gather": (c_int, [_P, c_int64, c_int64, _P, c_int64, _P, _P]),
     "esr_segreduce": (c_int, [c_int, c_int, _P, c_int64, _P, _P, c_int64, _P, _P]),
+    "esr_linsys_apply": (c_int, [c_int, _P, _P, _P, _P, _P, _P, c_int64, _P, _P]),
     "esr_aggregate_workspace_bytes": (c_int64, [c_int64, c_int64]),
     "esr_aggregate": (c_int, [c_int, c_int, _P, c_int64, c_int64, _P, _P, _P]),
     "esr_aggregate_noalloc": (c_int, [c_int, c_int, _P, c_int64, c_int64, _P, _P]),

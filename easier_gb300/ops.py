@@ -9,6 +9,7 @@ from __future__ import annotations
 from typing import Optional
 
 import torch
+from torch.nn.modules import module as _nn_module
 
 from . import _lib
 from .utils import EasierJitException
@@ -69,6 +70,46 @@ def reduce(red, tensor: torch.Tensor, out: Optional[torch.Tensor] = None) -> tor
     if dst is not out:
         out.copy_(dst)
     return out
+
+
+def _plain_call(mod) -> bool:
+    """Calling ``mod`` runs its class's forward and nothing else."""
+    return "forward" not in mod.__dict__ and not (mod._forward_hooks or mod._forward_pre_hooks or mod._backward_hooks
+                                                  or mod._backward_pre_hooks)
+
+
+def _observed() -> bool:
+    """Something watches torch operations (modes, tracing, forward-mode AD,
+    vmap, global module hooks): fused paths would hide them."""
+    C = torch._C
+    return bool(C._len_torch_dispatch_stack() or C._len_torch_function_stack() or C._get_tracing_state() is not None
+                or torch.autograd.forward_ad._current_level >= 0 or C._functorch.maybe_current_level() is not None
+                or torch.compiler.is_compiling()
+                or _nn_module._global_forward_hooks or _nn_module._global_forward_pre_hooks
+                or _nn_module._global_backward_hooks or _nn_module._global_backward_pre_hooks)
+
+
+def linsys_apply(A, x: torch.Tensor) -> Optional[torch.Tensor]:
+    """reducer(selector(x) * Ae) + x * Av in one kernel (esr_linsys_apply,
+    bitwise the five-step form), or None where the five steps could do
+    anything else: other shapes and dtypes (broadcasts, promotion), gradients,
+    hooks, subclasses, an index out of range."""
+    from .module import Reducer, Selector, Tensor
+    sel, red, Ae, Av = A.selector, A.reducer, A.Ae, A.Av
+    if type(sel) is not Selector or type(red) is not Reducer or red.reduce != "sum"             or sel.easier_index_status != "rewritten" or red.easier_index_status != "rewritten"             or not _plain_call(sel) or not _plain_call(red) or _observed():
+        return None
+    for t in (x, Ae, Av):
+        if type(t) not in (torch.Tensor, torch.nn.Parameter, Tensor) or t.dim() != 1 or t.dtype != x.dtype                 or t.device != x.device or (t.requires_grad and torch.is_grad_enabled()):
+            return None
+    n, m = red.n, red._perm32.shape[0]
+    if x.dtype not in (torch.float32, torch.float64) or x.device.type != "cuda" or x.layout is not torch.strided             or x.shape[0] != n or Av.shape[0] != n or Ae.shape[0] != m or sel._idx32.shape[0] != m             or sel._idx_max >= n or sel._idx32.device != x.device or red._perm32.device != x.device             or not Ae.is_contiguous() or not Av.is_contiguous():
+        return None
+    x = x.contiguous()
+    y = torch.empty_like(x, requires_grad=False)
+    _lib.call("esr_linsys_apply", _lib.dtype_code(x.dtype), _lib.ptr(x), _lib.ptr(Ae), _lib.ptr(Av),
+              _lib.ptr(sel._idx32), _lib.ptr(red._rowptr32), _perm_ptr(red), n, _lib.ptr(y),
+              _lib.stream_handle(x.device))
+    return y
 
 
 _AGG = {"sum": _lib.AGG_SUM, "prod": _lib.AGG_PROD, "norm": _lib.AGG_NORM, "max": _lib.AGG_MAX, "min": _lib.AGG_MIN}

@@ -213,6 +213,18 @@ int esr_segreduce(int dtype, int op, const void *t, int64_t row_elems,
                   const int32_t *rowptr, const int32_t *perm, int64_t n,
                   void *out, void *stream);
 
+/* y = A x of a Linsys in one pass:
+ *   y[i] = (sum over k in [rowptr[i], rowptr[i+1]) of x[col[e]] * ae[e],
+ *           e = perm ? perm[k] : k, ascending k) + x[i] * av[i]
+ * with every product and sum rounded on its own, i.e. bitwise
+ * reducer(selector(x) * Ae) + x * Av (easier/numeric/linsys.py:23-24).
+ * col: the Selector's index; rowptr, perm: the Reducer's CSR (perm NULL =
+ * the edges already lie in row order).  x and y [n] do not overlap; every
+ * col value lies in [0, n) (the caller has checked).  dtype ESR_F32/F64. */
+int esr_linsys_apply(int dtype, const void *x, const void *ae, const void *av,
+                     const int32_t *col, const int32_t *rowptr,
+                     const int32_t *perm, int64_t n, void *y, void *stream);
+
 /* Bytes of scratch esr_aggregate needs for an [n, cols] input. */
 int64_t esr_aggregate_workspace_bytes(int64_t n, int64_t cols);
 

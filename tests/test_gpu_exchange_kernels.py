@@ -7,6 +7,8 @@ import pytest
 import torch
 
 import easier_gb300 as esr
+from easier_gb300 import _lib, ops
+from easier_gb300.numeric import Linsys
 from oracle import sparse as osp
 
 pytestmark = pytest.mark.gpu
@@ -79,3 +81,42 @@ def test_segments(op, dtype, cols):
         empty = torch.bincount(i, minlength=n) == 0
         assert torch.equal(kept[empty], out[empty]) and int(empty.sum()) >= 2
         assert np.array_equal(kept[~empty].numpy(), want[~empty].numpy(), equal_nan=dtype.is_floating_point)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("n,m,shuffled", [(1, 0, False), (255, 900, True), (256, 2048, False), (257, 5001, True),
+                                          (70_001, 400_000, True)])
+def test_linsys_apply_is_bitwise_the_five_operations(dtype, n, m, shuffled):
+    g = torch.Generator().manual_seed(n)
+    row = torch.randint(0, n, (m,), generator=g)
+    row = row if shuffled else row.sort().values
+    col = torch.randint(0, n, (m,), generator=g)
+
+    class M(esr.Module):
+        def __init__(self):
+            super().__init__()
+            self.sel, self.red = esr.Selector(col), esr.Reducer(row, n)
+            self.Ae = esr.Tensor(torch.randn(m, generator=g).to(dtype), mode="partition")
+            self.Av = esr.Tensor(torch.randn(n, generator=g).to(dtype), mode="partition")
+            self.A = Linsys(self.Av, self.Ae, self.sel, self.red)
+
+    mod = M()
+    esr.compile([mod], "cuda")
+    x = torch.randn(n, generator=g).to(dtype)
+    x[n // 2] = -0.0
+    wide = torch.stack([x, x], 1).cuda()
+    for v in (x.cuda(), wide[:, 0]):  # contiguous and strided
+        fused = ops.linsys_apply(mod.A, v)
+        assert fused is not None
+        want = mod.red(mod.sel(v) * mod.Ae) + v * mod.Av
+        assert torch.equal(fused, want) and torch.equal(mod.A(v), want)
+    if m and dtype == torch.float64:
+        bad = x.cuda()
+        bad[0] = float("inf")
+        want = mod.red(mod.sel(bad) * mod.Ae) + bad * mod.Av
+        assert np.array_equal(mod.A(bad).cpu().numpy(), want.cpu().numpy(), equal_nan=True)
+        # what the kernel does not cover keeps the five operations
+        assert ops.linsys_apply(mod.A, x.float().cuda()) is None
+        assert mod.A(x.float().cuda()).dtype == torch.float64
+        v = x.cuda().requires_grad_()
+        assert ops.linsys_apply(mod.A, v) is None and mod.A(v).requires_grad
