@@ -450,141 +450,245 @@ int launch_linsys(const void *x, const void *ae, const void *av, const int32_t *
 }
 
 // ---------------------------------------------------------- aggregate --
-// Two launches: blocks reduce fixed row ranges into partials, then one
-// block per column reduces the partials in block order.
-constexpr int64_t kAggRowsPerBlock = 8192;
-constexpr int kAggMaxBlocks = 1024;
+// Two launches (one for short inputs): blocks reduce strided parts into
+// partials, then one block per column reduces the partials in block order.
+// Bound: HBM / L2 for max and min, the FP64 pipe (one DADD or DFMA a value)
+// for sums.  Extrema are taken on order-preserving integer keys: a double
+// compare costs the FP64 pipe what an add does, integer compares run beside
+// it.  A block covers kAggUnroll * W values at a time, W the largest multiple
+// of `cols` up to kThreads, so a thread stays in one column of coalesced,
+// independent loads.  8 M doubles: sum 31 -> 22 us, norm 48 -> 20, max 67 ->
+// 16 (first launch, cold cache); the final launch's latency (6 us alone) is
+// hidden in part by launching it early.
+constexpr int kAggUnroll = 8;
+constexpr int kAggMaxBlocks = 152 * 4;
+constexpr int64_t kAggSingle = 8192;  // values one block takes alone: the second launch costs more
 
-int64_t agg_blocks(int64_t n) {
-  int64_t b = (n + kAggRowsPerBlock - 1) / kAggRowsPerBlock;
-  if (b < 1) b = 1;
-  if (b > kAggMaxBlocks) b = kAggMaxBlocks;
-  return b;
-}
-
-template <typename T>
-struct AggTraits {
-  using acc_t = double;
-};
-template <>
-struct AggTraits<int32_t> {
-  using acc_t = int64_t;
-};
-template <>
-struct AggTraits<int64_t> {
-  using acc_t = int64_t;
-};
+// acc_t A: load(T) -> A, combine(A, A), identity(), store(A) -> T
+template <typename T, int AGG>
+struct Agg;
 
 template <typename A, int AGG>
-__device__ __forceinline__ A agg_identity() {
-  if (AGG == ESR_AGG_PROD) return A(1);
-  if (AGG == ESR_AGG_MAX || AGG == ESR_AGG_MIN) return A(0);  // replaced by first value
-  return A(0);
-}
-
-template <typename A, int AGG>
-__device__ __forceinline__ A agg_combine(A a, A b, bool a_valid) {
-  if (!a_valid) {
-    if (AGG == ESR_AGG_SUM || AGG == ESR_AGG_NORM) return b;
-    if (AGG == ESR_AGG_PROD) return b;
-    return b;
+struct AggSum {  // sum, prod, norm in A = double (floating T) or int64
+  static __device__ __forceinline__ A identity() { return AGG == ESR_AGG_PROD ? A(1) : A(0); }
+  static __device__ __forceinline__ A combine(A a, A b) {
+    return AGG == ESR_AGG_PROD ? ops<A>::mul(a, b) : ops<A>::add(a, b);
   }
-  if (AGG == ESR_AGG_SUM || AGG == ESR_AGG_NORM) return ops<A>::add(a, b);
-  if (AGG == ESR_AGG_PROD) return ops<A>::mul(a, b);
-  if (AGG == ESR_AGG_MAX) return is_nan(b) ? b : (is_nan(a) ? a : ((a < b) ? b : a));
-  return is_nan(b) ? b : (is_nan(a) ? a : ((b < a) ? b : a));
-}
+};
 
-// Block-wide fixed-order combine of one value per thread; result in lane 0
-// of warp 0.  `valid` marks threads that saw at least one element.
-template <typename A, int AGG>
-__device__ A block_combine(A v, bool valid, bool &any_valid) {
-  __shared__ A s_val[kThreads];
-  __shared__ int s_ok[kThreads];
-  s_val[threadIdx.x] = v;
-  s_ok[threadIdx.x] = valid ? 1 : 0;
+template <typename T, int AGG>
+struct AggFloat : AggSum<double, AGG> {
+  using A = double;
+  static __device__ __forceinline__ A add(A a, T v) {
+    if (AGG == ESR_AGG_NORM) return fma((double)v, (double)v, a);
+    return AggSum<double, AGG>::combine(a, (double)v);
+  }
+  static __device__ __forceinline__ T store(A a) { return (T)(AGG == ESR_AGG_NORM ? sqrt(a) : a); }
+};
+
+// bits of a float / double -> signed integers in the values' order, every
+// NaN at the end that wins (max: the top, min: the bottom)
+template <typename I, typename U, int AGG>
+struct AggKey {
+  using A = I;
+  static constexpr I kMag = (I)(~(U)0 >> 1);
+  static constexpr I kLow = (I)((U)1 << (8 * sizeof(U) - 1));
+  static constexpr I kWin = AGG == ESR_AGG_MAX ? kMag : kLow;
+  static __device__ __forceinline__ I identity() { return AGG == ESR_AGG_MAX ? kLow : kMag; }
+  static __device__ __forceinline__ I combine(I a, I b) {
+    return AGG == ESR_AGG_MAX ? (a < b ? b : a) : (b < a ? b : a);
+  }
+  static __device__ __forceinline__ I key(I bits, U inf) {
+    const I k = bits ^ ((bits >> (8 * sizeof(I) - 1)) & kMag);
+    return ((U)bits << 1) > (inf << 1) ? kWin : k;
+  }
+  static __device__ __forceinline__ I bits(I k) { return k ^ ((k >> (8 * sizeof(I) - 1)) & kMag); }
+};
+
+template <int AGG>
+struct AggExtF64 : AggKey<int64_t, uint64_t, AGG> {
+  using K = AggKey<int64_t, uint64_t, AGG>;
+  static __device__ __forceinline__ int64_t add(int64_t a, double v) {
+    return K::combine(a, K::key(__double_as_longlong(v), 0x7ff0000000000000ull));
+  }
+  static __device__ __forceinline__ double store(int64_t k) { return __longlong_as_double(K::bits(k)); }
+};
+
+template <int AGG>
+struct AggExtF32 : AggKey<int32_t, uint32_t, AGG> {
+  using K = AggKey<int32_t, uint32_t, AGG>;
+  static __device__ __forceinline__ int32_t add(int32_t a, float v) {
+    return K::combine(a, K::key(__float_as_int(v), 0x7f800000u));
+  }
+  static __device__ __forceinline__ float store(int32_t k) { return __int_as_float(K::bits(k)); }
+};
+
+template <typename T, int AGG>
+struct AggInt : AggSum<int64_t, AGG> {
+  using A = int64_t;
+  static __device__ __forceinline__ A add(A a, T v) { return AggSum<int64_t, AGG>::combine(a, (int64_t)v); }
+  static __device__ __forceinline__ T store(A a) { return (T)a; }
+};
+
+template <typename T, int AGG>
+struct AggIntExt : AggKey<int64_t, uint64_t, AGG> {
+  static __device__ __forceinline__ int64_t add(int64_t a, T v) {
+    return AggKey<int64_t, uint64_t, AGG>::combine(a, (int64_t)v);
+  }
+  static __device__ __forceinline__ T store(int64_t a) { return (T)a; }
+};
+
+constexpr bool is_ext(int agg) { return agg == ESR_AGG_MAX || agg == ESR_AGG_MIN; }
+template <bool C, class X, class Y>
+struct Pick { using type = X; };
+template <class X, class Y>
+struct Pick<false, X, Y> { using type = Y; };
+template <int AGG>
+struct Agg<float, AGG> : Pick<is_ext(AGG), AggExtF32<AGG>, AggFloat<float, AGG>>::type {};
+template <int AGG>
+struct Agg<double, AGG> : Pick<is_ext(AGG), AggExtF64<AGG>, AggFloat<double, AGG>>::type {};
+template <int AGG>
+struct Agg<int32_t, AGG> : Pick<is_ext(AGG), AggIntExt<int32_t, AGG>, AggInt<int32_t, AGG>>::type {};
+template <int AGG>
+struct Agg<int64_t, AGG> : Pick<is_ext(AGG), AggIntExt<int64_t, AGG>, AggInt<int64_t, AGG>>::type {};
+
+// Combines the accumulators of threads t, t + w, t + 2w, ... < rows * w into
+// thread t < w.  One column: the first warp adds eight values a lane, then
+// shuffles (13 adds a block where a shuffle tree over eight warps issues 45;
+// the FP64 pipe is the bound of sums).
+template <class G>
+__device__ __forceinline__ typename G::A agg_block(typename G::A acc, int rows, int w, typename G::A *s) {
+  const int t = threadIdx.x;
+  s[t] = acc;
   __syncthreads();
-  for (int w = kThreads / 2; w > 0; w >>= 1) {
-    if ((int)threadIdx.x < w) {
-      const int o = threadIdx.x + w;
-      if (s_ok[o]) {
-        s_val[threadIdx.x] = agg_combine<A, AGG>(s_val[threadIdx.x], s_val[o], s_ok[threadIdx.x] != 0);
-        s_ok[threadIdx.x] = 1;
-      }
+  if (w == 1) {
+    if (t < 32) {
+      for (int k = 32; k < kThreads; k += 32) acc = G::combine(acc, s[t + k]);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) acc = G::combine(acc, __shfl_down_sync(0xffffffffu, acc, o));
     }
+    return acc;
+  }
+  int top = 1;
+  while (top < rows) top <<= 1;
+  for (int h = top >> 1; h > 0; h >>= 1) {
+    if (t < h * w && t + h * w < rows * w) s[t] = G::combine(s[t], s[t + h * w]);
     __syncthreads();
   }
-  A r = s_val[0];
-  any_valid = s_ok[0] != 0;
-  __syncthreads();
-  return r;
+  return s[t < w ? t : 0];
 }
 
+// blocks x columns: partial[b * cols + c]; a single block stores the result
 template <typename T, int AGG>
-__global__ void __launch_bounds__(kThreads)
-agg_partial_kernel(const T *__restrict__ t, int64_t n, int64_t cols, int64_t rows_per_block,
-                   typename AggTraits<T>::acc_t *__restrict__ partial, int *__restrict__ partial_ok) {
-  using A = typename AggTraits<T>::acc_t;
-  const int64_t r0 = (int64_t)blockIdx.x * rows_per_block;
-  int64_t r1 = r0 + rows_per_block;
-  if (r1 > n) r1 = n;
-  for (int64_t c = 0; c < cols; ++c) {
-    A acc = agg_identity<A, AGG>();
-    bool valid = false;
-    for (int64_t r = r0 + threadIdx.x; r < r1; r += blockDim.x) {
-      A v = (A)t[r * cols + c];
-      if (AGG == ESR_AGG_NORM) v = ops<A>::mul(v, v);
-      acc = agg_combine<A, AGG>(acc, v, valid);
-      valid = true;
-    }
-    bool any = false;
-    A tot = block_combine<A, AGG>(acc, valid, any);
-    if (threadIdx.x == 0) {
-      partial[(int64_t)blockIdx.x * cols + c] = tot;
-      partial_ok[(int64_t)blockIdx.x * cols + c] = any ? 1 : 0;
-    }
+__global__ void __launch_bounds__(kThreads, 4)
+agg_partial_kernel(const T *__restrict__ t, int64_t n, int64_t cols, typename Agg<T, AGG>::A *__restrict__ partial,
+                   T *__restrict__ out) {
+  using G = Agg<T, AGG>;
+  __shared__ typename G::A s[kThreads];
+  cudaTriggerProgrammaticLaunchCompletion();  // the final launch may queue up; it waits for this grid's end
+  typename G::A acc = G::identity();
+  int rows = 1, w = kThreads;
+  int64_t c = threadIdx.x;
+  if (cols <= kThreads) {
+    w = (int)cols;
+    rows = kThreads / w;
+    const int64_t W = (int64_t)rows * w, total = n * cols, step = (int64_t)gridDim.x * kAggUnroll * W;
+    if ((int)threadIdx.x < W)
+      for (int64_t base = (int64_t)blockIdx.x * kAggUnroll * W + threadIdx.x; base < total; base += step) {
+        T v[kAggUnroll];
+#pragma unroll
+        for (int u = 0; u < kAggUnroll; ++u)
+          if (base + u * W < total) v[u] = t[base + u * W];
+#pragma unroll
+        for (int u = 0; u < kAggUnroll; ++u)
+          if (base + u * W < total) acc = G::add(acc, v[u]);
+      }
+  } else {  // wide rows: one column a thread, kThreads columns a block (blockIdx.y)
+    c += (int64_t)blockIdx.y * kThreads;
+    const int64_t step = (int64_t)gridDim.x * kAggUnroll;
+    if (c < cols)
+      for (int64_t r = (int64_t)blockIdx.x * kAggUnroll; r < n; r += step) {
+        T v[kAggUnroll];
+#pragma unroll
+        for (int u = 0; u < kAggUnroll; ++u)
+          if (r + u < n) v[u] = t[(r + u) * cols + c];
+#pragma unroll
+        for (int u = 0; u < kAggUnroll; ++u)
+          if (r + u < n) acc = G::add(acc, v[u]);
+      }
   }
+  const typename G::A tot = agg_block<G>(acc, rows, w, s);
+  if ((int)threadIdx.x >= w || c >= cols) return;
+  // (empty input: sum and norm 0, prod 1; the host rejects empty max / min)
+  if (gridDim.x == 1) out[c] = n > 0 || !is_ext(AGG) ? G::store(tot) : T(0);
+  else partial[(int64_t)blockIdx.x * cols + c] = tot;
 }
 
 template <typename T, int AGG>
 __global__ void __launch_bounds__(kThreads)
-agg_final_kernel(const typename AggTraits<T>::acc_t *__restrict__ partial, const int *__restrict__ partial_ok,
-                 int64_t nblocks, int64_t cols, T *__restrict__ out) {
-  using A = typename AggTraits<T>::acc_t;
+agg_final_kernel(const typename Agg<T, AGG>::A *__restrict__ partial, int nblocks, int64_t cols,
+                 T *__restrict__ out) {
+  using G = Agg<T, AGG>;
+  __shared__ typename G::A s[kThreads];
+  cudaGridDependencySynchronize();
   const int64_t c = blockIdx.x;
-  A acc = agg_identity<A, AGG>();
-  bool valid = false;
-  for (int64_t b = threadIdx.x; b < nblocks; b += blockDim.x) {
-    if (partial_ok[b * cols + c]) {
-      acc = agg_combine<A, AGG>(acc, partial[b * cols + c], valid);
-      valid = true;
-    }
+  typename G::A acc = G::identity();
+#pragma unroll 4
+  for (int b = threadIdx.x; b < nblocks; b += kThreads) acc = G::combine(acc, partial[b * cols + c]);
+  const typename G::A tot = agg_block<G>(acc, kThreads, 1, s);
+  if (threadIdx.x == 0) out[c] = G::store(tot);
+}
+
+// Scratch a call may be asked for by the static array's limit (one slot of
+// 12 bytes per column and 8,192 rows, at most 1,024)
+int64_t agg_limit_bytes(int64_t n, int64_t cols) {
+  int64_t b = (n + 8191) / 8192;
+  b = b < 1 ? 1 : b > 1024 ? 1024 : b;
+  return b * (cols < 1 ? 1 : cols) * 12;
+}
+
+// Row blocks of the first launch: enough values each to pay for a block, at
+// most four blocks an SM, and partials within ESR_AGG_NOALLOC_SCRATCH_BYTES
+// or what the limit above already allows.
+int64_t agg_blocks(int64_t n, int64_t cols) {
+  if (cols < 1) cols = 1;
+  if (n * cols <= kAggSingle) return 1;
+  int64_t b;
+  if (cols <= kThreads) {
+    const int64_t per = (int64_t)kAggUnroll * (kThreads / cols) * cols;
+    b = (n * cols + per - 1) / per;
+  } else {
+    b = (n + kAggUnroll - 1) / kAggUnroll;
+    const int64_t fill = kAggMaxBlocks / ((cols + kThreads - 1) / kThreads);
+    if (b > fill) b = fill;
   }
-  bool any = false;
-  A tot = block_combine<A, AGG>(acc, valid, any);
-  if (threadIdx.x == 0) {
-    if (!any) {
-      // empty input: sum/norm -> 0, prod -> 1, max/min -> NaN (torch raises;
-      // the host rejects empty max/min before calling)
-      if (AGG == ESR_AGG_PROD) tot = A(1);
-      else tot = A(0);
-    }
-    if (AGG == ESR_AGG_NORM) out[c] = (T)sqrt((double)tot);
-    else out[c] = (T)tot;
-  }
+  if (b > kAggMaxBlocks) b = kAggMaxBlocks;
+  int64_t room = (int64_t)ESR_AGG_NOALLOC_SCRATCH_BYTES;
+  if (agg_limit_bytes(n, cols) > room) room = agg_limit_bytes(n, cols);
+  if (b > room / (8 * cols)) b = room / (8 * cols);
+  return b < 1 ? 1 : b;
 }
 
 template <typename T, int AGG>
 int launch_agg_t(const void *t, int64_t n, int64_t cols, void *out, void *ws, cudaStream_t st) {
-  using A = typename AggTraits<T>::acc_t;
-  const int64_t nb = agg_blocks(n);
-  const int64_t rpb = (n + nb - 1) / nb;
+  using A = typename Agg<T, AGG>::A;
+  const int64_t nb = agg_blocks(n, cols);
+  const unsigned gy = cols <= kThreads ? 1u : (unsigned)((cols + kThreads - 1) / kThreads);
   A *partial = (A *)ws;
-  int *ok = (int *)((char *)ws + nb * cols * sizeof(double));
-  agg_partial_kernel<T, AGG><<<(int)nb, kThreads, 0, st>>>((const T *)t, n, cols, rpb < 1 ? 1 : rpb, partial, ok);
+  agg_partial_kernel<T, AGG><<<dim3((unsigned)nb, gy), kThreads, 0, st>>>((const T *)t, n, cols, partial, (T *)out);
   ESR_LAUNCH_CHECK("esr_aggregate/partial");
-  agg_final_kernel<T, AGG><<<(int)cols, kThreads, 0, st>>>(partial, ok, nb, cols, (T *)out);
-  ESR_LAUNCH_CHECK("esr_aggregate/final");
+  if (nb == 1) return ESR_OK;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)cols);
+  cfg.blockDim = dim3(kThreads);
+  cfg.stream = st;
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, agg_final_kernel<T, AGG>, (const A *)partial, (int)nb, cols, (T *)out);
+  if (e != cudaSuccess) return esr::cuda_check(e, "esr_aggregate/final");
   return ESR_OK;
 }
 
@@ -593,7 +697,9 @@ int launch_agg(int agg, const void *t, int64_t n, int64_t cols, void *out, void 
   switch (agg) {
     case ESR_AGG_SUM: return launch_agg_t<T, ESR_AGG_SUM>(t, n, cols, out, ws, st);
     case ESR_AGG_PROD: return launch_agg_t<T, ESR_AGG_PROD>(t, n, cols, out, ws, st);
-    case ESR_AGG_NORM: return launch_agg_t<T, ESR_AGG_NORM>(t, n, cols, out, ws, st);
+    case ESR_AGG_NORM:
+      if constexpr (sizeof(T) == 0 || T(0.5) == T(0)) return esr::fail(ESR_ERR_UNSUPPORTED, "norm of an integer tensor");
+      else return launch_agg_t<T, ESR_AGG_NORM>(t, n, cols, out, ws, st);
     case ESR_AGG_MAX: return launch_agg_t<T, ESR_AGG_MAX>(t, n, cols, out, ws, st);
     case ESR_AGG_MIN: return launch_agg_t<T, ESR_AGG_MIN>(t, n, cols, out, ws, st);
     default: return esr::fail(ESR_ERR_ARG, "unknown aggregator");
@@ -678,7 +784,8 @@ extern "C" int esr_linsys_apply(int dtype, const void *x, const void *ae, const 
 
 extern "C" int64_t esr_aggregate_workspace_bytes(int64_t n, int64_t cols) {
   if (n < 0 || cols < 0) return -1;
-  return agg_blocks(n) * (cols < 1 ? 1 : cols) * (int64_t)(sizeof(double) + sizeof(int));
+  const int64_t limit = agg_limit_bytes(n, cols), need = agg_blocks(n, cols) * (cols < 1 ? 1 : cols) * 8;
+  return need > limit ? need : limit;
 }
 
 extern "C" int esr_aggregate(int dtype, int agg, const void *t, int64_t n, int64_t cols, void *out,
@@ -791,7 +898,7 @@ extern "C" int esr_aggregate_noalloc(int dtype, int agg, const void *t, int64_t 
   if (n < 0 || cols < 0) return esr::fail(ESR_ERR_ARG, "esr_aggregate_noalloc: negative size");
   if (cols == 0) return ESR_OK;
   if (!out || (n && !t)) return esr::fail(ESR_ERR_ARG, "esr_aggregate_noalloc: null pointer");
-  const int64_t need = esr_aggregate_workspace_bytes(n, cols);
+  const int64_t need = agg_limit_bytes(n, cols);
   if (need > (int64_t)ESR_AGG_NOALLOC_SCRATCH_BYTES)
     return esr::fail(ESR_ERR_ARG, "esr_aggregate_noalloc: n=" + std::to_string(n) + ", cols=" +
                                       std::to_string(cols) + " needs " + std::to_string(need) +

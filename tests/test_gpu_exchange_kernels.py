@@ -120,3 +120,45 @@ def test_linsys_apply_is_bitwise_the_five_operations(dtype, n, m, shuffled):
         assert mod.A(x.float().cuda()).dtype == torch.float64
         v = x.cuda().requires_grad_()
         assert ops.linsys_apply(mod.A, v) is None and mod.A(v).requires_grad
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64, torch.int32, torch.int64])
+@pytest.mark.parametrize("n,cols", [(1, 1), (8192, 1), (8193, 1), (1_000_003, 1), (5000, 2), (40_001, 3), (300, 64),
+                                    (2049, 255), (777, 256), (777, 257), (9, 1000)])
+def test_aggregates(dtype, n, cols):
+    g = torch.Generator().manual_seed(n + cols)
+    t = torch.randn(n, *(() if cols == 1 else (cols,)), generator=g, dtype=torch.float64)
+    t = (t if dtype.is_floating_point else t * 1000).to(dtype)
+    c, d = t.cuda(), t.double()
+    assert torch.equal(esr.max(c).cpu(), t.amax(0, keepdim=True))
+    assert torch.equal(esr.min(c).cpu(), t.amin(0, keepdim=True))
+    if not dtype.is_floating_point:
+        assert torch.equal(esr.sum(c).cpu(), t.sum(0, keepdim=True).to(dtype))
+        return
+    ulp = torch.finfo(dtype).eps
+    bound = n * 2.0 ** -53 * d.abs().sum(0, keepdim=True)
+    want = d.sum(0, keepdim=True)
+    assert bool(((esr.sum(c).cpu().double() - want).abs() <= bound + ulp * want.abs()).all())
+    want = d.norm(dim=0, keepdim=True)
+    assert bool(((esr.norm(c).cpu().double() - want).abs() <= (n * 2.0 ** -53 + 2 * ulp) * want).all())
+    assert torch.equal(esr.sum(c), esr.sum(c))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+def test_extrema_of_special_values(dtype):
+    lo, hi = -torch.finfo(dtype).max, torch.finfo(dtype).max
+    inf, nan = float("inf"), float("nan")
+    for vals, mx, mn in (([-inf, -inf], -inf, -inf), ([lo, -inf], lo, -inf), ([inf, hi], inf, hi), ([-1.0, nan], nan, nan),
+                         ([-nan, 2.0], nan, nan), ([-0.0, -0.0], 0.0, 0.0), ([5e-45, -5e-45], 5e-45, -5e-45)):
+        for n in (2, 20_000):
+            t = torch.tensor(vals, dtype=dtype).repeat(n // 2).cuda()
+            for got, want in ((esr.max(t), mx), (esr.min(t), mn)):
+                want = torch.tensor([want], dtype=dtype)
+                assert np.array_equal(got.cpu().numpy(), want.numpy(), equal_nan=True), (vals, n)
+
+
+def test_empty_aggregates():
+    t = torch.zeros(0, 3, dtype=torch.float64, device="cuda")
+    assert torch.equal(esr.sum(t).cpu(), torch.zeros(1, 3, dtype=torch.float64))
+    assert torch.equal(ops.aggregate(t, "prod").cpu(), torch.ones(1, 3, dtype=torch.float64))
+    assert ops.device_status(clear=True) & _lib.DEV_IDX_RANGE == 0
