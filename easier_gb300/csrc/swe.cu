@@ -35,10 +35,12 @@
 //   4: D4 = delta(S1);           s0 = s0 + c4*(A + D4)
 #include <algorithm>
 #include <cstdint>
+#include <type_traits>
 #include <vector>
 
 #include "esr_internal.h"
 #include "reduce_util.cuh"
+#include "soft64.cuh"
 
 namespace {
 
@@ -55,8 +57,19 @@ struct Ar<T, true> {
   static __device__ __forceinline__ T sub(T a, T b) { return O::sub(a, b); }
   // a*b + c, two roundings
   static __device__ __forceinline__ T madd(T a, T b, T c) { return O::add(O::mul(a, b), c); }
-  static __device__ __forceinline__ T recip(T) { return T(0); }
-  static __device__ __forceinline__ T quot(T x, T y, T) { return O::div(x, y); }
+  // a divisor shared by several quotients.  Double: prepared once for the
+  // integer division of soft64.cuh, the machine's quotient bit for bit; the
+  // nine FP64 divisions of a cell were 44% of the exact stage's FP64-pipe time
+  // (627 -> 382 us a stage at 1.97 M cells, FP64 pipe 83% either way)
+  struct Plain {
+    T y;
+  };
+  using Div = std::conditional_t<std::is_same<T, double>::value, soft64::Divisor, Plain>;
+  static __device__ __forceinline__ Div divisor(T y) { return Div{y}; }
+  static __device__ __forceinline__ T quot(T x, const Div &d) {
+    if constexpr (std::is_same<T, double>::value) return soft64::quotient(x, d);
+    else return O::div(x, d.y);
+  }
 };
 
 template <>
@@ -71,7 +84,6 @@ struct Ar<float, false> {
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(y));
     return r;
   }
-  static __device__ __forceinline__ float quot(float x, float, float yinv) { return x * yinv; }
 };
 
 template <>
@@ -80,8 +92,7 @@ struct Ar<double, false> {
   static __device__ __forceinline__ double add(double a, double b) { return a + b; }
   static __device__ __forceinline__ double sub(double a, double b) { return a - b; }
   static __device__ __forceinline__ double madd(double a, double b, double c) { return fma(a, b, c); }
-  static __device__ __forceinline__ double recip(double y) { return 1.0 / y; }
-  static __device__ __forceinline__ double quot(double x, double, double yinv) { return x * yinv; }
+  static __device__ __forceinline__ double recip(double y) { return soft64::quotient(1.0, soft64::Divisor(y)); }
 };
 
 template <typename T>
@@ -113,25 +124,25 @@ __device__ __forceinline__ void add_face(Acc3<T> &s, T oh, T ou, T ov, T nh, T n
     s.Sh = A::add(s.Sh, Fh);
     s.Su = A::madd(uhf, Fi, A::madd(hfs, fx, s.Su));
     s.Sv = A::madd(vhf, Fi, A::madd(hfs, fy, s.Sv));
-    return;
+  } else {
+    const T half = T(0.5);
+    const T om = A::sub(T(1), a);
+    const T hf = A::madd(om, nh, A::mul(a, oh));   // (1 - alpha)*h[src] + alpha*h[dst]
+    const T uhf = A::madd(om, nu, A::mul(a, ou));
+    const T vhf = A::madd(om, nv, A::mul(a, ov));
+    const auto by_hf = A::divisor(hf);
+    const T uf = A::quot(uhf, by_hf);
+    const T vf = A::quot(vhf, by_hf);
+    const T hfs = A::mul(A::mul(half, hf), hf);    // 0.5 * h_f * h_f
+    const T uhsx = A::mul(uhf, fx);                // uh_f * sx
+    const T vhsy = A::mul(vhf, fy);                // vh_f * sy
+    const T Fh = A::add(uhsx, vhsy);
+    const T Fu = A::madd(A::madd(uf, uhf, hfs), fx, A::mul(uf, vhsy));
+    const T Fv = A::madd(vf, uhsx, A::mul(A::madd(vf, vhf, hfs), fy));
+    s.Sh = A::add(s.Sh, Fh);
+    s.Su = A::add(s.Su, Fu);
+    s.Sv = A::add(s.Sv, Fv);
   }
-  const T half = T(0.5);
-  const T om = A::sub(T(1), a);
-  const T hf = A::madd(om, nh, A::mul(a, oh));   // (1 - alpha)*h[src] + alpha*h[dst]
-  const T uhf = A::madd(om, nu, A::mul(a, ou));
-  const T vhf = A::madd(om, nv, A::mul(a, ov));
-  const T ih = A::recip(hf);
-  const T uf = A::quot(uhf, hf, ih);
-  const T vf = A::quot(vhf, hf, ih);
-  const T hfs = A::mul(A::mul(half, hf), hf);    // 0.5 * h_f * h_f
-  const T uhsx = A::mul(uhf, fx);                // uh_f * sx
-  const T vhsy = A::mul(vhf, fy);                // vh_f * sy
-  const T Fh = A::add(uhsx, vhsy);
-  const T Fu = A::madd(A::madd(uf, uhf, hfs), fx, A::mul(uf, vhsy));
-  const T Fv = A::madd(vf, uhsx, A::mul(A::madd(vf, vhf, hfs), fy));
-  s.Sh = A::add(s.Sh, Fh);
-  s.Su = A::add(s.Su, Fu);
-  s.Sv = A::add(s.Sv, Fv);
 }
 
 // A wall face: 0.5 * gather_b(h)**2 * (bsx, bsy)
@@ -152,13 +163,15 @@ __device__ __forceinline__ void add_wall(Acc3<T> &s, T oh, T fx, T fy) {
 template <typename T, bool EXACT>
 __device__ __forceinline__ void finish(const Acc3<T> &s, T ar, T iar, T &dh, T &du, T &dv) {
   using A = Ar<T, EXACT>;
-  dh = A::quot(-s.Sh, ar, iar);
   if constexpr (EXACT) {
-    du = A::quot(-A::add(s.Su, s.Bu), ar, iar);
-    dv = A::quot(-A::add(s.Sv, s.Bv), ar, iar);
+    const auto by_area = A::divisor(ar);
+    dh = A::quot(-s.Sh, by_area);
+    du = A::quot(-A::add(s.Su, s.Bu), by_area);
+    dv = A::quot(-A::add(s.Sv, s.Bv), by_area);
   } else {  // wall terms are in Su, Sv
-    du = A::quot(-s.Su, ar, iar);
-    dv = A::quot(-s.Sv, ar, iar);
+    dh = -s.Sh * iar;
+    du = -s.Su * iar;
+    dv = -s.Sv * iar;
   }
 }
 
