@@ -1,12 +1,13 @@
-// IEEE double division on the integer and FP32 pipes.
+// IEEE double division and multiplication on the integer and FP32 pipes.
 //
 // GB300's FP64 pipe runs 1/59 of its FP32 rate: one FP64 instruction of a
-// warp holds a scheduler's share of the pipe for about 64 cycles, and a
-// division issues eight or nine of them.  The same quotient, correctly
-// rounded, takes about 45 integer instructions, which the other pipes run in
-// a sixth of that time.
+// warp holds a scheduler's share of the pipe for 64 cycles, and a division
+// issues eight or nine of them.  The same quotient, correctly rounded, takes
+// about 45 integer instructions, which the other pipes run in a sixth of that
+// time; a product about 45 too, no faster than the machine's, but beside it:
+// a kernel bound by the FP64 pipe runs part of its products here.
 //
-// Method: long division with a 32-bit reciprocal (Knuth, TAOCP vol. 2, 4.3.1:
+// Division: long division with a 32-bit reciprocal (Knuth, TAOCP vol. 2, 4.3.1:
 // a digit estimated from below and corrected by its remainder).  With
 // mantissas ma, mb in [2^52, 2^53), ma doubled if below mb, the quotient
 // ma / mb lies in [1, 2):
@@ -149,6 +150,95 @@ ESR_HD double quotient(double a, const Divisor &d) {
   if (plain) return value(out);
   const bool zero = (ua << 1) == 0 && (uint32_t)(eb - 1) < 2046u;  // 0 / normal
   return zero ? value(sign) : a / d.b;
+}
+
+// a * b, rounded to nearest even.  A = 2^11 ma times mb has its 53 result bits
+// in the product's upper 64 (one fewer if ma mb < 2^105: all three words move
+// up by s) and the fraction to round by in the lower 64.
+ESR_HD uint32_t shift_left(uint32_t lo, uint32_t hi, uint32_t s) {  // upper word of hi:lo << s
+#ifdef __CUDA_ARCH__
+  return __funnelshift_l(lo, hi, s);
+#else
+  return (uint32_t)((((uint64_t)hi << 32 | lo) << s) >> 32);
+#endif
+}
+
+// The machine's product for rare paths, kept out of line: inlined, the
+// compiler predicates the one instruction, which then takes the FP64 pipe of
+// warps that do not need it.
+#ifdef __CUDACC__
+static __host__ __device__ __noinline__
+#else
+inline
+#endif
+double machine_product(double a, double b) {
+#ifdef __CUDA_ARCH__
+  return __dmul_rn(a, b);
+#else
+  return a * b;
+#endif
+}
+
+// (mh:ml:t) + r, with e added to the upper word
+ESR_HD void round_up(uint32_t &mh, uint32_t &ml, uint32_t t, uint32_t r, uint32_t e) {
+#ifdef __CUDA_ARCH__
+  asm("{\n.reg .u32 d;\nadd.cc.u32 d, %2, %3;\naddc.cc.u32 %1, %1, 0;\naddc.u32 %0, %0, %4;\n}\n"
+      : "+r"(mh), "+r"(ml)
+      : "r"(t), "r"(r), "r"(e));
+#else
+  const uint32_t c = (uint32_t)(((uint64_t)t + r) >> 32);
+  const uint64_t m = ((uint64_t)mh << 32 | ml) + c;
+  mh = (uint32_t)(m >> 32) + e;
+  ml = (uint32_t)m;
+#endif
+}
+
+ESR_HD double product(double a, double b) {
+  const uint64_t ua = bits(a), ub = bits(b);
+  const uint32_t ha = (uint32_t)(ua >> 32), la = (uint32_t)ua, hb = (uint32_t)(ub >> 32), lb = (uint32_t)ub;
+  // both exponents' top two bits differ: factors within 2^-511 .. 2^512
+  if (((ha ^ (ha << 1)) & (hb ^ (hb << 1)) & 0x40000000u) != 0) {
+    const uint32_t ah = shift_left(la, ha, 11) | 0x80000000u, al = la << 11;
+    const uint32_t bh = (hb & 0xfffffu) | 0x100000u;
+    const uint64_t p00 = (uint64_t)al * lb;
+    const uint64_t p01 = (uint64_t)al * bh + (p00 >> 32);
+    const uint64_t p10 = (uint64_t)ah * lb + (uint32_t)p01;
+    const uint64_t p11 = (uint64_t)ah * bh + (p01 >> 32) + (p10 >> 32);
+    uint32_t mh = (uint32_t)(p11 >> 32), ml = (uint32_t)p11, f1 = (uint32_t)p10, f0 = (uint32_t)p00;
+    const uint32_t s = ((mh >> 20) & 1u) ^ 1u;
+    mh = shift_left(ml, mh, s);
+    ml = shift_left(f1, ml, s);
+    f1 = shift_left(f0, f1, s);
+    f0 <<= s;
+    const uint32_t t = f1 | (f0 != 0 ? 1u : 0u);
+    // the leading bit of the mantissa adds one to the exponent field
+    const uint32_t e = (ha & 0x7ff00000u) + (hb & 0x7ff00000u) - (1023u << 20) + s * 0xfff00000u;
+    round_up(mh, ml, t, 0x7fffffffu + (ml & 1u), e);
+    return value((uint64_t)(mh | ((ha ^ hb) & 0x80000000u)) << 32 | ml);
+  }
+  const bool za = (ua << 1) == 0, zb = (ub << 1) == 0;
+  const bool fa = (ha & 0x7ff00000u) != 0x7ff00000u, fb = (hb & 0x7ff00000u) != 0x7ff00000u;
+  if ((za && fb) || (zb && fa)) return value((ua ^ ub) & 0x8000000000000000ull);
+  return machine_product(a, b);
+}
+
+// a / 2: one less in the exponent field (subnormal results: the machine's)
+ESR_HD double half(double a) {
+  const uint64_t u = bits(a);
+  const uint32_t e = (uint32_t)(u >> 52) & 0x7ffu;
+  if (e - 2u < 2045u) return value(u - 0x0010000000000000ull);
+  return machine_product(a, 0.5);
+}
+
+// -a without the FP64 add the compiler makes of it
+ESR_HD double negated(double a) { return value(bits(a) ^ 0x8000000000000000ull); }
+
+// 0 + a: a, with -0 turned into +0
+ESR_HD double from_zero(double a) {
+  const uint64_t u = bits(a);
+  const uint32_t hi = (uint32_t)(u >> 32), lo = (uint32_t)u;
+  const uint32_t kept = ((hi << 1) | lo) == 0 ? 0u : hi;
+  return value((uint64_t)kept << 32 | lo);
 }
 
 }  // namespace soft64

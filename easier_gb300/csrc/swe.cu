@@ -45,6 +45,7 @@
 namespace {
 
 constexpr int kSweThreads = 256;
+constexpr int kStageThreads = 128;
 
 template <typename T, bool EXACT>
 struct Ar;
@@ -53,6 +54,25 @@ template <typename T>
 struct Ar<T, true> {
   using O = ops<T>;
   static __device__ __forceinline__ T mul(T a, T b) { return O::mul(a, b); }
+  // the same product on the integer pipes (double)
+  static __device__ __forceinline__ T imul(T a, T b) {
+    if constexpr (std::is_same<T, double>::value) return soft64::product(a, b);
+    else return O::mul(a, b);
+  }
+  static __device__ __forceinline__ T imadd(T a, T b, T c) { return O::add(imul(a, b), c); }
+  static __device__ __forceinline__ T neg(T a) {
+    if constexpr (std::is_same<T, double>::value) return soft64::negated(a);
+    else return -a;
+  }
+  // 0 + a
+  static __device__ __forceinline__ T from_zero(T a) {
+    if constexpr (std::is_same<T, double>::value) return soft64::from_zero(a);
+    else return O::add(T(0), a);
+  }
+  static __device__ __forceinline__ T half(T a) {
+    if constexpr (std::is_same<T, double>::value) return soft64::half(a);
+    else return O::mul(T(0.5), a);
+  }
   static __device__ __forceinline__ T add(T a, T b) { return O::add(a, b); }
   static __device__ __forceinline__ T sub(T a, T b) { return O::sub(a, b); }
   // a*b + c, two roundings
@@ -78,6 +98,7 @@ struct Ar<float, false> {
   static __device__ __forceinline__ float add(float a, float b) { return a + b; }
   static __device__ __forceinline__ float sub(float a, float b) { return a - b; }
   static __device__ __forceinline__ float madd(float a, float b, float c) { return fmaf(a, b, c); }
+  static __device__ __forceinline__ float imadd(float a, float b, float c) { return fmaf(a, b, c); }
   // approximate reciprocal (one MUFU op, ~1 ulp; flushes subnormals)
   static __device__ __forceinline__ float recip(float y) {
     float r;
@@ -92,6 +113,7 @@ struct Ar<double, false> {
   static __device__ __forceinline__ double add(double a, double b) { return a + b; }
   static __device__ __forceinline__ double sub(double a, double b) { return a - b; }
   static __device__ __forceinline__ double madd(double a, double b, double c) { return fma(a, b, c); }
+  static __device__ __forceinline__ double imadd(double a, double b, double c) { return fma(a, b, c); }
   static __device__ __forceinline__ double recip(double y) { return soft64::quotient(1.0, soft64::Divisor(y)); }
 };
 
@@ -111,7 +133,8 @@ struct Acc3 {
 //          F_vh  = (vh_f / h_f) F_h + h_f^2 / 2 sy
 //          (u_f uh_f sx + u_f vh_f sy = u_f F_h), each term an FMA into the
 //          sum, and the wall terms go straight into the same sums.
-template <typename T, bool EXACT>
+// FIRST: the sums are still zero.
+template <typename T, bool EXACT, bool FIRST = false>
 __device__ __forceinline__ void add_face(Acc3<T> &s, T oh, T ou, T ov, T nh, T nu, T nv, T a, T fx, T fy) {
   using A = Ar<T, EXACT>;
   if constexpr (!EXACT) {
@@ -125,23 +148,28 @@ __device__ __forceinline__ void add_face(Acc3<T> &s, T oh, T ou, T ov, T nh, T n
     s.Su = A::madd(uhf, Fi, A::madd(hfs, fx, s.Su));
     s.Sv = A::madd(vhf, Fi, A::madd(hfs, fy, s.Sv));
   } else {
-    const T half = T(0.5);
     const T om = A::sub(T(1), a);
-    const T hf = A::madd(om, nh, A::mul(a, oh));   // (1 - alpha)*h[src] + alpha*h[dst]
-    const T uhf = A::madd(om, nu, A::mul(a, ou));
-    const T vhf = A::madd(om, nv, A::mul(a, ov));
+    const T hf = A::imadd(om, nh, A::imul(a, oh));   // (1 - alpha)*h[src] + alpha*h[dst]
+    const T uhf = A::imadd(om, nu, A::imul(a, ou));
+    const T vhf = A::imadd(om, nv, A::imul(a, ov));
     const auto by_hf = A::divisor(hf);
     const T uf = A::quot(uhf, by_hf);
     const T vf = A::quot(vhf, by_hf);
-    const T hfs = A::mul(A::mul(half, hf), hf);    // 0.5 * h_f * h_f
+    const T hfs = A::imul(A::half(hf), hf);        // 0.5 * h_f * h_f
     const T uhsx = A::mul(uhf, fx);                // uh_f * sx
     const T vhsy = A::mul(vhf, fy);                // vh_f * sy
     const T Fh = A::add(uhsx, vhsy);
-    const T Fu = A::madd(A::madd(uf, uhf, hfs), fx, A::mul(uf, vhsy));
-    const T Fv = A::madd(vf, uhsx, A::mul(A::madd(vf, vhf, hfs), fy));
-    s.Sh = A::add(s.Sh, Fh);
-    s.Su = A::add(s.Su, Fu);
-    s.Sv = A::add(s.Sv, Fv);
+    const T Fu = A::madd(A::imadd(uf, uhf, hfs), fx, A::imul(uf, vhsy));
+    const T Fv = A::imadd(vf, uhsx, A::mul(A::imadd(vf, vhf, hfs), fy));
+    if constexpr (FIRST) {
+      s.Sh = A::from_zero(Fh);
+      s.Su = A::from_zero(Fu);
+      s.Sv = A::from_zero(Fv);
+    } else {
+      s.Sh = A::add(s.Sh, Fh);
+      s.Su = A::add(s.Su, Fu);
+      s.Sv = A::add(s.Sv, Fv);
+    }
   }
 }
 
@@ -161,13 +189,21 @@ __device__ __forceinline__ void add_wall(Acc3<T> &s, T oh, T fx, T fy) {
 
 // delta = -(sums) / area
 template <typename T, bool EXACT>
-__device__ __forceinline__ void finish(const Acc3<T> &s, T ar, T iar, T &dh, T &du, T &dv) {
+__device__ __forceinline__ void finish(const Acc3<T> &s, bool walls, T ar, T iar, T &dh, T &du, T &dv) {
   using A = Ar<T, EXACT>;
   if constexpr (EXACT) {
     const auto by_area = A::divisor(ar);
-    dh = A::quot(-s.Sh, by_area);
-    du = A::quot(-A::add(s.Su, s.Bu), by_area);
-    dv = A::quot(-A::add(s.Sv, s.Bv), by_area);
+    dh = A::quot(A::neg(s.Sh), by_area);
+    T tu, tv;  // (without wall faces Bu and Bv are zero)
+    if (std::is_same<T, double>::value && !walls) {
+      tu = A::from_zero(s.Su);
+      tv = A::from_zero(s.Sv);
+    } else {
+      tu = A::add(s.Su, s.Bu);
+      tv = A::add(s.Sv, s.Bv);
+    }
+    du = A::quot(A::neg(tu), by_area);
+    dv = A::quot(A::neg(tv), by_area);
   } else {  // wall terms are in Su, Sv
     dh = -s.Sh * iar;
     du = -s.Su * iar;
@@ -208,33 +244,54 @@ struct SlotsG {  // face slots in global memory, [width][nc]
 };
 
 // delta (swe_main.py:87-119) of cell i given the stage state `s`.
+template <typename T, int W, bool EXACT, bool FIRST>
+__device__ __forceinline__ void slot_sums(int k, int64_t i, int64_t nc, const SlotsG<T> &g, const T *s,
+                                          const Vec4<T> own, Acc3<T> &acc, bool &walls) {
+  const int32_t j = __ldg(g.nbr + k * nc + i);
+  if (j >= 0) {
+    if ((int64_t)j >= nc) {  // corrupt slot: flag it, never read out of bounds
+      esr::raise_status(ESR_DEV_IDX_RANGE);
+      return;
+    }
+    const Vec4<T> nb = load4(s + 4 * (int64_t)j);
+    add_face<T, EXACT, FIRST>(acc, own.x, own.y, own.z, nb.x, nb.y, nb.z, __ldg(g.alpha + k * nc + i),
+                              __ldg(g.sx + k * nc + i), __ldg(g.sy + k * nc + i));
+  } else if (j == -1) {
+    add_wall<T, EXACT>(acc, own.x, __ldg(g.sx + k * nc + i), __ldg(g.sy + k * nc + i));
+    walls = true;
+  }
+}
+
 template <typename T, int W, bool EXACT>
 __device__ __forceinline__ Vec4<T> cell_delta(int64_t i, int64_t nc, const SlotsG<T> &g, const T *s,
                                               const Vec4<T> own) {
   Acc3<T> acc{T(0), T(0), T(0), T(0), T(0)};
+  bool walls = false;
+  slot_sums<T, W, EXACT, true>(0, i, nc, g, s, own, acc, walls);
+  if constexpr (EXACT && std::is_same<T, double>::value) {
+    // (one copy of the long integer code: unrolled, the stage's instructions
+    // no longer stay in the instruction cache)
+#pragma unroll 1
+    for (int k = 1; k < W; ++k) slot_sums<T, W, EXACT, false>(k, i, nc, g, s, own, acc, walls);
+  } else {
 #pragma unroll
-  for (int k = 0; k < W; ++k) {
-    const int32_t j = __ldg(g.nbr + k * nc + i);
-    if (j >= 0) {
-      if ((int64_t)j >= nc) {  // corrupt slot: flag it, never read out of bounds
-        esr::raise_status(ESR_DEV_IDX_RANGE);
-        continue;
-      }
-      const Vec4<T> nb = load4(s + 4 * (int64_t)j);
-      add_face<T, EXACT>(acc, own.x, own.y, own.z, nb.x, nb.y, nb.z, __ldg(g.alpha + k * nc + i),
-                         __ldg(g.sx + k * nc + i), __ldg(g.sy + k * nc + i));
-    } else if (j == -1) {
-      add_wall<T, EXACT>(acc, own.x, __ldg(g.sx + k * nc + i), __ldg(g.sy + k * nc + i));
-    }
+    for (int k = 1; k < W; ++k) slot_sums<T, W, EXACT, false>(k, i, nc, g, s, own, acc, walls);
   }
   Vec4<T> d;
-  finish<T, EXACT>(acc, __ldg(g.area + i), EXACT ? T(0) : __ldg(g.inv_area + i), d.x, d.y, d.z);
+  finish<T, EXACT>(acc, walls, __ldg(g.area + i), EXACT ? T(0) : __ldg(g.inv_area + i), d.x, d.y, d.z);
   d.w = T(0);
   return d;
 }
 
+// Exact FP64 is bound by the FP64 pipe and, beside it, the integer pipe: of a
+// face's 16 products four (by sx, sy, often exactly zero) and the twelve adds
+// stay on the FP64 pipe, the rest and every division run as integer work
+// (soft64.cuh).  1.97 M cells: 627 us a stage with all of it on the FP64 pipe
+// (87% busy), 382 with integer divisions, 300 with eleven integer products a
+// face, 241 with one copy of the face code, no adds to zero and 128-thread
+// CTAs (FP64 pipe 73%, integer pipe 61%); all products as integers: 325.
 template <typename T, int W, int STAGE, bool EXACT>
-__global__ void __launch_bounds__(kSweThreads)
+__global__ void __launch_bounds__(kStageThreads, 8)
 swe_stage_kernel(int64_t nc, SlotsG<T> g, const T *__restrict__ sin, const T *s0, T *__restrict__ acc, T *sout,
                  T c) {
   using A = Ar<T, EXACT>;
@@ -245,9 +302,9 @@ swe_stage_kernel(int64_t nc, SlotsG<T> g, const T *__restrict__ sin, const T *s0
   const Vec4<T> base = (STAGE == 1) ? own_in : load4(s0 + 4 * i);
   Vec4<T> out;
   if (STAGE < 4) {
-    out.x = A::madd(c, d.x, base.x);
-    out.y = A::madd(c, d.y, base.y);
-    out.z = A::madd(c, d.z, base.z);
+    out.x = A::imadd(c, d.x, base.x);
+    out.y = A::imadd(c, d.y, base.y);
+    out.z = A::imadd(c, d.z, base.z);
     out.w = T(0);
     Vec4<T> a;
     if (STAGE == 1) {
@@ -296,10 +353,16 @@ SlotsG<T> slots_of(const esr_swe_mesh *m) {
                    (const T *)m->inv_area};
 }
 
+// CTA size of a stage launch: small meshes take 64-thread CTAs, so that no SM
+// gets a 256-cell CTA more than another (40,000 cells: 157 CTAs of 256 leave
+// five SMs with twice the others' work).
+int stage_threads(int64_t nc) { return nc < (int64_t)152 * 16 * kStageThreads ? 64 : kStageThreads; }
+
 template <typename T, int W, bool EXACT>
 int run_steps(const esr_swe_mesh *m, double dt, T *state, int64_t steps, T *ws, cudaStream_t st) {
   const int64_t nc = m->nc;
-  const int grid = (int)((nc + kSweThreads - 1) / kSweThreads);
+  const int threads = stage_threads(nc);
+  const int grid = (int)((nc + threads - 1) / threads);
   T *S1 = ws;
   T *S2 = ws + 4 * nc;
   T *A = ws + 8 * nc;
@@ -310,10 +373,10 @@ int run_steps(const esr_swe_mesh *m, double dt, T *state, int64_t steps, T *ws, 
   const T c3 = (T)dt;
   const T c4 = (T)(dt / 6);
   for (int64_t s = 0; s < steps; ++s) {
-    swe_stage_kernel<T, W, 1, EXACT><<<grid, kSweThreads, 0, st>>>(nc, g, state, state, A, S1, c1);
-    swe_stage_kernel<T, W, 2, EXACT><<<grid, kSweThreads, 0, st>>>(nc, g, S1, state, A, S2, c1);
-    swe_stage_kernel<T, W, 3, EXACT><<<grid, kSweThreads, 0, st>>>(nc, g, S2, state, A, S1, c3);
-    swe_stage_kernel<T, W, 4, EXACT><<<grid, kSweThreads, 0, st>>>(nc, g, S1, state, A, state, c4);
+    swe_stage_kernel<T, W, 1, EXACT><<<grid, threads, 0, st>>>(nc, g, state, state, A, S1, c1);
+    swe_stage_kernel<T, W, 2, EXACT><<<grid, threads, 0, st>>>(nc, g, S1, state, A, S2, c1);
+    swe_stage_kernel<T, W, 3, EXACT><<<grid, threads, 0, st>>>(nc, g, S2, state, A, S1, c3);
+    swe_stage_kernel<T, W, 4, EXACT><<<grid, threads, 0, st>>>(nc, g, S1, state, A, state, c4);
   }
   ESR_LAUNCH_CHECK("esr_swe_step");
   return ESR_OK;
@@ -453,7 +516,7 @@ __device__ __forceinline__ void tile_delta(int j, const CellGeom &c, int nL, con
     }
   }
   if (EXACT) {
-    finish<float, true>(acc, c.area, 0.f, dh, du, dv);
+    finish<float, true>(acc, true, c.area, 0.f, dh, du, dv);
   } else {  // the area is in the records, the wall terms in Su, Sv
     dh = -acc.Sh;
     du = -acc.Su;

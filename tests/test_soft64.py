@@ -52,6 +52,9 @@ int main() {
     const float bh = fvalue((((hi << 3) | (lo >> 29)) & 0x7fffffu) | 0x3f800000u);
     d.r = reciprocal(hi, lo, fvalue(fbits(1.0f / bh) + (uint32_t)(rnd() % 5) - 2u));
     if (!same(quotient(a, d), a / b) && bad++ < 5) std::printf("%a / %a\n", a, b);
+    if (!same(product(a, b), a * b) && bad++ < 5) std::printf("%a * %a\n", a, b);
+    if (!same(half(a), a * 0.5) && bad++ < 5) std::printf("%a / 2\n", a);
+    if (!same(from_zero(a), 0.0 + a) && bad++ < 5) std::printf("0 + %a\n", a);
   }
   std::printf("bad %ld\n", bad);
   return bad != 0;
@@ -59,7 +62,7 @@ int main() {
 """
 
 
-def test_integer_division_is_the_machines(tmp_path):
+def test_integer_arithmetic_is_the_machines(tmp_path):
     cxx = shutil.which("g++")
     if cxx is None:
         pytest.skip("no C++ compiler")
