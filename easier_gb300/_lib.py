@@ -141,6 +141,9 @@ _SIGS = {
     "esr_bcg_workspace_bytes": (c_int64, [c_int32, c_int32, c_int32]),
     "esr_bcg_init": (c_int, [POINTER(Batch), _P, _P, _P, _P, _P, _P, c_double, c_double, c_int32, _P, _P]),
     "esr_bcg_iterate": (c_int, [POINTER(Batch), _P, _P, _P, _P, _P, c_int32, _P, _P]),
+    "esr_pcg_solo_ctas": (c_int, [POINTER(Batch)]),
+    "esr_pcg_solo_comm_bytes": (c_int64, []),
+    "esr_pcg_solo_iterate": (c_int, [POINTER(Batch), c_int32, _P, _P, _P, _P, _P, c_int32, _P, _P, _P]),
     "esr_bcg_verify": (c_int, [POINTER(Batch), _P, _P, _P, _P, _P, _P, _P, _P, _P]),
     "esr_bcg_status": (c_int, [_P, c_int32, c_int32, POINTER(c_int32), POINTER(BcgInst), _P]),
     "esr_gnn_apply": (c_int, [POINTER(Batch), _P, _P, _P, _P]),

@@ -175,6 +175,11 @@ def chunk_layout(inst_block0: np.ndarray, tiles_per_chunk: int):
 GNN_STALL_WINDOW = 16
 
 
+# iterations of one single-system launch at most (it stops by itself; this
+# bounds how long the host waits for a launch)
+SOLO_ITERS = 4096
+
+
 class BatchedPCG:
     """Lockstep (P)CG over a packed batch on one GPU.
 
@@ -264,7 +269,15 @@ class BatchedPCG:
                                      _lib.ptr(g["layer_w"]), _lib.ptr(g["layer_b"]), _lib.ptr(g["dec_w"]),
                                      float(gnn.dec_b), int(gnn_ctas_per_sm * self.sm_count),
                                      int(GNN_STALL_WINDOW if stall_window is None else stall_window), 0)
+        self._solo_comm = None
         self.set_shape(tiles_per_chunk, grid if grid is not None else 4 * self.sm_count)
+        # one FP64 system whose vectors fit the chip: iterations inside one
+        # cooperative launch (the work shape then only matters to solve_graph)
+        with torch.cuda.device(dev):
+            self.solo = int(_lib.lib().esr_pcg_solo_ctas(ctypes.byref(self.desc))) > 0
+        if self.solo:
+            self._solo_width = int(np.diff(pk.slice_ptr).max()) // 32
+            self._solo_comm = torch.zeros(int(_lib.lib().esr_pcg_solo_comm_bytes()), dtype=torch.uint8, device=dev)
 
     def set_shape(self, tiles_per_chunk: int, grid: int):
         """Work unit of the persistent kernels (tiles per chunk) and their
@@ -316,6 +329,12 @@ class BatchedPCG:
     def _iterate_call(self, k: int):
         _lib.call("esr_bcg_iterate", ctypes.byref(self.desc), _lib.ptr(self.x), _lib.ptr(self.r), _lib.ptr(self.z),
                   _lib.ptr(self.p), _lib.ptr(self.q), int(k), _lib.ptr(self.ws), self._stream())
+
+    def _solo_group(self, k: int):
+        self.kernel_launches += 1
+        _lib.call("esr_pcg_solo_iterate", ctypes.byref(self.desc), self._solo_width, _lib.ptr(self.x), _lib.ptr(self.r),
+                  _lib.ptr(self.z), _lib.ptr(self.p), _lib.ptr(self.q), int(k), _lib.ptr(self.ws),
+                  _lib.ptr(self._solo_comm), self._stream())
 
     def _group(self, k: int):
         per_it = (2 if self.precision == "df64" else 3) + (5 if self.gnn_desc is not None else 0) + self.poly_degree
@@ -439,13 +458,14 @@ class BatchedPCG:
             max_rounds: int = 16) -> int:
         """Device part of a solve; returns the number of verification rounds."""
         self.start(rtol, atol, maxiter)
-        k = min(8, self.graph_iters)
+        group, most = (self._solo_group, SOLO_ITERS) if self.solo else (self._group, self.graph_iters)
+        k = min(64 if self.solo else 8, most)
         rounds = 0
         while True:
             active = self.active()
             while active > 0:
-                self._group(k)
-                k = min(self.graph_iters, 2 * k)
+                group(k)
+                k = min(most, 2 * k)
                 active = self.active()
             self.verify()
             rounds += 1
@@ -503,7 +523,13 @@ class BatchedPCG:
         step() calls - 1), the final recurrence residual, the FP64 true
         residual and the number of residual replacements."""
         self.run(rtol, atol, maxiter, max_rounds)
-        return [self._info(s) for s in self.instances()]
+        insts = self.instances()
+        if self.solo and insts[0].done == 3:
+            from .. import ops
+            if ops.device_status(clear=True) & _lib.DEV_WAIT_TIMEOUT:
+                self._solo_comm.zero_()
+                raise RuntimeError("the CTAs of a CG launch timed out waiting for one another")
+        return [self._info(s) for s in insts]
 
     @staticmethod
     def _info(s) -> dict:

@@ -154,7 +154,8 @@ class CG(esr.Module):
                                       A.Ae.data, A.Av.data, self.b.data)
                 eng = BatchedPCG([inst], jacobi=jacobi, precision="df64" if precision == "df64" else "fp64",
                                  device=self.x.device)
-                eng.autotune()
+                if not eng.solo:
+                    eng.autotune()
                 return eng
             return FusedPCG(SellMatrix.from_linsys(A), jacobi=jacobi)
 

@@ -740,6 +740,23 @@ int esr_bcg_init(const esr_batch *B, const double *b64, const void *b, void *x,
 int esr_bcg_iterate(const esr_batch *B, void *x, void *r, void *z, void *p,
                     void *q, int32_t k, void *workspace, void *stream);
 
+/* Iterations of a batch of one FP64 system (Jacobi or no preconditioner)
+ * whose vectors fit the multiprocessors' shared memory (about 1 M rows), as
+ * one cooperative launch of up to `k` iterations that keeps them there: the
+ * state, scalars and stopping test of esr_bcg_iterate, between which and
+ * this a solve must not switch (the first direction of a state that
+ * esr_bcg_init or esr_bcg_verify left is p = z; q = A z).
+ * esr_pcg_solo_ctas: the launch's CTAs on the current device, 0 if the batch
+ * does not qualify.  max_width: no slice has more slots (widest row).  comm: esr_pcg_solo_comm_bytes() of device memory, zeroed
+ * before its first use and used by one solve at a time.  CTAs wait for one
+ * another with a bounded poll; on time-out ESR_DEV_WAIT_TIMEOUT is raised,
+ * the instance stops (done = 3) and comm must be zeroed again. */
+int esr_pcg_solo_ctas(const esr_batch *B);
+int64_t esr_pcg_solo_comm_bytes(void);
+int esr_pcg_solo_iterate(const esr_batch *B, int32_t max_width, void *x,
+                         void *r, void *z, void *p, void *q, int32_t k,
+                         void *workspace, void *comm, void *stream);
+
 /* For every converged, unverified instance: x64 = x, r64 = b64 - A64 x64 in
  * FP64; verified = 1 when ||r64|| <= tol.  Otherwise r = r64 replaces the
  * recurrence residual (z = M r, and p = z + (r.z / r.z_old) p while
