@@ -155,6 +155,8 @@ _SIGS = {
     "esr_gmres_workspace_bytes": (c_int64, [c_int64, c_int32]),
     "esr_gmres_init": (c_int, [POINTER(Sell), _P, c_double, c_double, _P, _P]),
     "esr_gmres_residual": (c_int, [POINTER(Sell), _P, _P, _P, _P, _P]),
+    "esr_gmres_cycles": (c_int, [POINTER(Sell), _P, _P, _P, _P, _P, _P, c_int32, c_int32, _P, _P]),
+    "esr_gmres_one_launch": (c_int, [POINTER(Sell), c_int32]),
     "esr_gmres_cycle": (c_int, [POINTER(Sell), _P, _P, _P, _P, _P, _P, c_int32, _P, _P]),
     "esr_gmres_read": (c_int, [_P, POINTER(GmresScalars), _P]),
 }

@@ -172,7 +172,8 @@ class GMRES(esr.Module):
         use_fused = self.fusable() if fused is None else fused
         if use_fused:
             eng = self._fused_solver()
-            s, iters = eng.solve(self.b.data, self.x.data, self.r.data, rtol, atol, maxiter, log)
+            s, iters = eng.solve(self.b.data, self.x.data, self.r.data, rtol, atol, maxiter,
+                                 log if debug_iter is not None else None)
             rnorm, bnorm = float(s.rnorm), float(s.bnorm)
         else:
             rnorm, bnorm, iters = gmres_per_op(self.A, self.M, self.b.data, self.x.data, self.r.data,

@@ -241,10 +241,15 @@ class MixedPCG:
         return s
 
 
+# restart cycles of one launch at most (it stops by itself at the tolerance)
+GMRES_CYCLES = 16
+
+
 class FusedGMRES:
     """Restarted GMRES on a SELL matrix with M = Jacobi or identity
-    (gmres.py algorithm): one CUDA graph per restart cycle, one 64-byte read
-    of the device scalars per cycle for the host's stopping test."""
+    (gmres.py algorithm): one cooperative launch per restart cycle (or, for
+    systems it does not hold, one CUDA graph of many), one 64-byte read of the
+    device scalars per cycle for the host's stopping test."""
 
     def __init__(self, A: SellMatrix, restart: int, jacobi: bool = False, use_graph: bool = True):
         self.A = A
@@ -259,11 +264,15 @@ class FusedGMRES:
         self.ws = torch.zeros(nbytes, dtype=torch.uint8, device=self.dev)
         self.V = torch.empty((self.restart, self.n), dtype=self.dtype, device=self.dev)
         self.w2 = torch.empty((2, self.n), dtype=self.dtype, device=self.dev)
-        self.use_graph = use_graph
+        with torch.cuda.device(self.dev):
+            self.one_launch = bool(_lib.lib().esr_gmres_one_launch(ctypes.byref(A.desc), self.restart))
+        self.use_graph = use_graph and not self.one_launch
         self._graphs = {}
         self.kernel_launches = 0
 
     def launches_per_cycle(self) -> int:
+        if self.one_launch:
+            return 1
         R = self.restart
         return 1 + R + R * (R + 1) // 2 + 3
 
@@ -272,15 +281,15 @@ class FusedGMRES:
         _lib.call("esr_gmres_read", _lib.ptr(self.ws), ctypes.byref(out), _lib.stream_handle(self.dev))
         return out
 
-    def _cycle_call(self, b, x, r):
-        _lib.call("esr_gmres_cycle", ctypes.byref(self.A.desc), _lib.ptr(self.invdiag), _lib.ptr(b), _lib.ptr(x),
-                  _lib.ptr(r), _lib.ptr(self.V), _lib.ptr(self.w2), self.restart, _lib.ptr(self.ws),
+    def _cycle_call(self, b, x, r, cycles: int = 1):
+        _lib.call("esr_gmres_cycles", ctypes.byref(self.A.desc), _lib.ptr(self.invdiag), _lib.ptr(b), _lib.ptr(x),
+                  _lib.ptr(r), _lib.ptr(self.V), _lib.ptr(self.w2), self.restart, int(cycles), _lib.ptr(self.ws),
                   _lib.stream_handle(self.dev))
 
-    def _cycle(self, b, x, r):
+    def _cycle(self, b, x, r, cycles: int = 1):
         self.kernel_launches += self.launches_per_cycle()
         if not self.use_graph:
-            self._cycle_call(b, x, r)
+            self._cycle_call(b, x, r, cycles)
             return
         key = (b.data_ptr(), x.data_ptr(), r.data_ptr())
         g = self._graphs.get(key)
@@ -305,11 +314,16 @@ class FusedGMRES:
                   _lib.ptr(self.ws), st)
         self.kernel_launches += 2
         iters = 0
+        group = 1  # cycles a launch may run before the host looks again
         while True:
             s = self.scalars()
+            iters = int(s.cycles)
+            if s.broken == 2:
+                raise RuntimeError("the CTAs of a GMRES cycle timed out waiting for one another")
             if log is not None:
                 log(iters, s.rnorm)
             if (s.rnorm == s.rnorm and s.rnorm <= s.tol) or (maxiter is not None and iters >= maxiter):
                 return s, iters
-            iters += 1
-            self._cycle(b, x, r)
+            self._cycle(b, x, r, group if maxiter is None else min(group, maxiter - iters))
+            if self.one_launch and log is None:
+                group = min(2 * group, GMRES_CYCLES)

@@ -581,7 +581,8 @@ typedef struct {
   double bnorm;
   double tol;      /* max(rtol * bnorm, atol)                              */
   int32_t jend;    /* Arnoldi columns of the last cycle                    */
-  int32_t broken;  /* the last cycle stopped on H[j+1][j] < 1e-15          */
+  int32_t broken;  /* the last cycle stopped on H[j+1][j] < 1e-15; 2: its
+                      CTAs timed out waiting for one another               */
   int32_t cycles;  /* restart cycles run since esr_gmres_init             */
   int32_t pad_;
 } esr_gmres_scalars;
@@ -599,15 +600,25 @@ int esr_gmres_residual(const esr_sell *A, const void *b, const void *x, void *r,
                        void *workspace, void *stream);
 
 /* One restart cycle (gmres.py:245-261): V_0 = r / rnorm, `restart` Arnoldi
- * steps with modified Gram-Schmidt in the reference's order (stopping early
- * on H[j+1][j] < 1e-15), the Hessenberg least squares on the device (Givens
- * rotations; the reference's clamped SVD gives the same y for a full-rank
- * H), x += M (V y), then the residual for the next stopping test.  V is
- * [restart][n] (column-contiguous), w2 is [2][n] scratch.  A fixed launch
- * sequence: capturable in a CUDA graph. */
+ * steps with a Gram-Schmidt basis (stopping early on H[j+1][j] < 1e-15), the
+ * Hessenberg least squares on the device (Givens rotations; the reference's
+ * clamped SVD gives the same y for a full-rank H), x += M (V y), then the
+ * residual for the next stopping test.  V is [restart][n]
+ * (column-contiguous), w2 is [2][n] scratch.  Systems whose rows of w fit the
+ * multiprocessors' shared memory (esr_gmres_one_launch; about 3.7 M rows) run
+ * it as one cooperative launch with classical Gram-Schmidt applied twice,
+ * larger ones as a fixed launch sequence with modified Gram-Schmidt in the
+ * reference's order. */
+int esr_gmres_one_launch(const esr_sell *A, int32_t restart);
 int esr_gmres_cycle(const esr_sell *A, const void *invdiag, const void *b,
                     void *x, void *r, void *V, void *w2, int32_t restart,
                     void *workspace, void *stream);
+
+/* Up to `cycles` restart cycles, stopping after one whose rnorm is at most
+ * tol; more than one needs esr_gmres_one_launch. */
+int esr_gmres_cycles(const esr_sell *A, const void *invdiag, const void *b,
+                     void *x, void *r, void *V, void *w2, int32_t restart,
+                     int32_t cycles, void *workspace, void *stream);
 
 /* Copy the scalars to host memory (synchronises `stream`). */
 int esr_gmres_read(const void *workspace, esr_gmres_scalars *out, void *stream);
