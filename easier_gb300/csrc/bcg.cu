@@ -17,13 +17,16 @@
 // p.q) and the update sweep (x, r, z, r.r, r.z), plus the GNN layers and a
 // z fix-up in GNN batches.  The double-float policy forms the direction in
 // one sweep (q = A z + beta q); the FP64 policy, bound by the FP64 pipe,
-// keeps q = A p and a separate p-update sweep at the end of the iteration.  A one-CTA compaction
-// kernel at the start of every esr_bcg_iterate call lists the chunks of the
+// keeps q = A p and a separate p-update sweep at the end of the iteration.  A
+// one-CTA compaction kernel at the start of every esr_bcg_iterate call lists the chunks of the
 // instances still running, so finished instances cost nothing afterwards.
+// The double-float direction sweep and the update sweep stream their tiles
+// through shared memory (bcg_stream.cuh).
 // Each dot product is finished per instance by the instance's last chunk to
-// arrive (atomic ticket), which adds the instance's chunk partials in chunk
-// order: deterministic, no floating-point atomics, no CTA ever waits for
-// another.
+// arrive (atomic ticket), which adds the instance's chunk partials in a fixed
+// order: deterministic, no floating-point atomics.  No CTA waits for another
+// to run; the streamed sweeps' last chunk may wait for sums that running CTAs
+// have already posted.
 //
 // Arithmetic policies:
 //   PolF64  FP64 vectors and matrix (the reference's precision);
@@ -43,9 +46,13 @@
 // residual misses the tolerance continues from it: r = b - A x replaces the
 // recurrence residual and p keeps its direction (a residual replacement,
 // not a restart).
+#include <algorithm>
+#include <cstring>
+#include <initializer_list>
 #include <vector>
 
 #include "bcg_common.cuh"
+#include "bcg_stream.cuh"
 
 namespace {
 
@@ -73,6 +80,10 @@ __global__ void __launch_bounds__(1024) bcg_compact_kernel(BArgs a, BcgLayout L)
     __syncthreads();
     if (threadIdx.x == 1023) s_base += s_scan[1023];
     __syncthreads();
+  }
+  for (int u = threadIdx.x; u < s_base; u += 1024) {
+    const int c = L.alist[u];
+    L.heads[u] = make_int4(c, a.chunk_inst[c], a.chunk_tile0[c], a.chunk_tile0[c + 1]);
   }
   if (threadIdx.x == 0) L.head->acount = s_base;
 }
@@ -143,45 +154,130 @@ bcg_init_kernel(BArgs a, const typename P::V *__restrict__ val, const typename P
 // A first direction (refresh != 0: after init or a residual replacement,
 // and the GNN's fallback to Jacobi) is p = z, q = A z.  The GNN's clipped
 // correction is folded into z by bcg_zfix_kernel before.
-template <class P>
-__global__ void __launch_bounds__(kBThreads, 4)
-bcg_pq_kernel(BArgs a, const typename P::V *__restrict__ val, const typename P::V *__restrict__ diag,
-              const typename P::V *__restrict__ z, typename P::V *__restrict__ p, typename P::V *__restrict__ q,
-              BcgLayout L) {
+// (Three CTAs a SM with two stages each: 24 warps compute; two with three or
+// four stages were slower.  A tile whose slices are wider than eight on average
+// reads its columns and values from memory.)
+constexpr int kPqCtas = 3, kUpdateCtas = 4;
+constexpr int kPqSlots = 8 * kBThreads;  // slots of a tile's slices that a stage has room for
+
+template <class P_>
+struct PqSweep {
+  using P = P_;
   using V = typename P::V;
-  const int count = L.head->acount;
-  for (int w = blockIdx.x; w < count; w += gridDim.x) {
-    const int c = L.alist[w];
-    const int inst = a.chunk_inst[c];
-    if (L.inst[inst].done) continue;
-    const bool first = L.inst[inst].refresh != 0;
-    const V beta = P::beta(L.inst[inst]);
-    typename P::Acc pq;
-    const int t1 = a.chunk_tile0[c + 1];
-#pragma unroll 2
-    for (int t = a.chunk_tile0[c]; t < t1; ++t) {
-      const int64_t i = (int64_t)t * kBThreads + threadIdx.x;
-      const V zi = z[i];
-      const V w = P::fma(diag[i], zi, bsell_row<P>(i, a.n, a.slice_ptr, a.col, val, z));
-      const V pi = first ? zi : P::fma(beta, p[i], zi);
-      const V qi = first ? w : P::fma(beta, q[i], w);
-      p[i] = pi;
-      q[i] = qi;
-      pq.add(pi, qi);
-    }
-    const double v[1] = {bsum<kBThreads>(pq)};
-    double tot[1];
-    if (chunk_finish<1>(a, c, inst, v, L, tot) && threadIdx.x == 0) {
-      esr_bcg_inst &s = L.inst[inst];
-      s.pq = tot[0];
-      if (!(tot[0] != 0.0) || !isfinite(tot[0])) {
-        s.done = 3;  // breakdown
-        retire(L);
-      } else {
-        set_alpha(s, s.rz / tot[0]);
+  static constexpr int S = 2, K = 1;
+  static constexpr uint32_t kSweep = 1;
+  static constexpr int kStageBytes = 4 * kTileBytes + 12 * kPqSlots;
+  struct Meta {
+    int64_t b;  // lane j <= 8: the first slot of slice j of the tile
+  };
+
+  const BArgs &a;
+  const V *__restrict__ val, *__restrict__ diag, *__restrict__ z;
+  V *__restrict__ p, *__restrict__ q;
+  bool wide;
+  typename P::Acc acc[1];
+
+  static __device__ __forceinline__ V coefficient(const esr_bcg_inst &s) { return P::beta(s); }
+  static __device__ __forceinline__ bool flag(const esr_bcg_inst &s) { return s.refresh != 0; }
+  __device__ __forceinline__ Meta meta(int t, int lane) const {
+    return Meta{lane <= kBWarps ? __ldg(a.slice_ptr + ((int64_t)t * kBWarps + lane)) : 0};
+  }
+  static __device__ __forceinline__ int slots_of(const Meta &m) {  // 0: they do not fit
+    const int64_t b0 = __shfl_sync(0xffffffffu, m.b, 0), slots = __shfl_sync(0xffffffffu, m.b, kBWarps) - b0;
+    return slots <= kPqSlots && !((slots | b0) & 31) ? (int)slots : 0;
+  }
+  // stage: z, diag, p, q, then the tile's columns and values if they fit
+  __device__ __forceinline__ void fetch(int t, const Meta &m, char *stage, int2 *slice, uint64_t *bar, int lane) const {
+    const int64_t i = (int64_t)t * kBThreads;
+    const int64_t b0 = __shfl_sync(0xffffffffu, m.b, 0);
+    const int64_t next = __shfl_down_sync(0xffffffffu, m.b, 1);
+    const int slots = slots_of(m), cb = 4 * slots;
+    // (where in the stage's slots the slice begins, and its width)
+    if (lane < kBWarps) slice[lane] = make_int2(slots ? (int)(m.b - b0) : -1, (int)((next - m.b) >> 5));
+    char *sc = stage + 4 * kTileBytes, *sv = sc + 4 * kPqSlots;
+    if (wide) {
+      __syncwarp();
+      if (lane == 0) {
+        bar_arrive_expect(bar, 4 * kTileBytes + 3 * cb);
+        if (cb) {
+          bulk_copy(sc, a.col + b0, cb, bar);
+          bulk_copy(sv, val + b0, 2 * cb, bar);
+        }
+        bulk_copy(stage, z + i, kTileBytes, bar);
+        bulk_copy(stage + kTileBytes, diag + i, kTileBytes, bar);
+        bulk_copy(stage + 2 * kTileBytes, p + i, kTileBytes, bar);
+        bulk_copy(stage + 3 * kTileBytes, q + i, kTileBytes, bar);
       }
+    } else {
+      plain_copy(stage, z + i, kTileBytes, lane);
+      plain_copy(stage + kTileBytes, diag + i, kTileBytes, lane);
+      plain_copy(stage + 2 * kTileBytes, p + i, kTileBytes, lane);
+      plain_copy(stage + 3 * kTileBytes, q + i, kTileBytes, lane);
+      plain_copy(sv, val + b0, 2 * cb, lane);
+      plain_copy(sc, a.col + b0, cb, lane);
+      __syncwarp();
+      if (lane == 0) bar_arrive(bar);
     }
   }
+  // sum + slots 0 .. 3 (those below w), in order
+  __device__ __forceinline__ V slots4(V sum, int w, const int32_t *cs, const V *vs) const {
+    int32_t c[4];
+    V x[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      c[k] = k < w ? cs[32 * k] : -1;
+      if ((int64_t)c[k] >= a.n) c[k] = -1;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (c[k] >= 0) x[k] = z[c[k]];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (c[k] >= 0) sum = P::fma(vs[32 * k], x[k], sum);
+    return sum;
+  }
+  __device__ __forceinline__ void compute(int t, const char *stage, int2 slice, V beta, int first) {
+    const int64_t i = (int64_t)t * kBThreads + threadIdx.x;
+    V sum = P::zero();
+    if (slice.x >= 0) {
+      const int at = slice.x + (threadIdx.x & 31);
+      const int32_t *cs = (const int32_t *)(stage + 4 * kTileBytes) + at;
+      const V *vs = (const V *)(stage + 4 * kTileBytes + 4 * kPqSlots) + at;
+      for (int k = 0; k < slice.y; k += 4) sum = slots4(sum, slice.y - k, cs + 32 * k, vs + 32 * k);
+    } else {
+      sum = bsell_row_of<P, false>(i, a.n, a.slice_ptr, a.col, val, [this](int64_t j) { return z[j]; });
+    }
+    const V *own = (const V *)stage + threadIdx.x;
+    const V zi = own[0];
+    const V w = P::fma(own[kBThreads], zi, sum);
+    const V pi = first ? zi : P::fma(beta, own[2 * kBThreads], zi);
+    const V qi = first ? w : P::fma(beta, own[3 * kBThreads], w);
+    p[i] = pi;
+    q[i] = qi;
+    acc[0].add(pi, qi);
+  }
+  BcgLayout L;
+  __device__ __forceinline__ void finish(esr_bcg_inst &s, const double (&tot)[1]) const {
+    s.pq = tot[0];
+    if (!(tot[0] != 0.0) || !isfinite(tot[0])) {
+      s.done = 3;  // breakdown
+      retire(L);
+    } else {
+      set_alpha(s, s.rz / tot[0]);
+    }
+  }
+};
+
+template <class P>
+__global__ void __launch_bounds__(kStreamThreads, kPqCtas)
+bcg_pq_kernel(BArgs a, const typename P::V *__restrict__ val, const typename P::V *__restrict__ diag,
+              const typename P::V *__restrict__ z, typename P::V *__restrict__ p, typename P::V *__restrict__ q,
+              bool wide, BcgLayout L) {
+  using OP = PqSweep<P>;
+  extern __shared__ __align__(128) char s_ring[];
+  __shared__ StreamShared<P, OP::S, OP::K> s_stream;
+  OP op{a, val, diag, z, p, q, wide, {}, L};
+  stream_chunks(a, L, s_ring, s_stream, op);
 }
 
 // ---- the same as two sweeps (FP64 policy): q = A p; p.q; alpha ...
@@ -270,74 +366,110 @@ bcg_zfix_kernel(BArgs a, const typename P::V *__restrict__ invdiag, const typena
 }
 
 // ---- step part 2 + update: x += a p; r -= a q; z = M r; r.r; r.z; test
-template <class P>
-__global__ void __launch_bounds__(kBThreads)
-bcg_update_kernel(BArgs a, const typename P::V *__restrict__ invdiag, typename P::V *__restrict__ x,
-                  typename P::V *__restrict__ r, typename P::V *__restrict__ z, const typename P::V *__restrict__ p,
-                  const typename P::V *__restrict__ q, BcgLayout L) {
+template <class P_>
+struct UpdateSweep {
+  using P = P_;
   using V = typename P::V;
-  const int count = L.head->acount;
-  for (int w = blockIdx.x; w < count; w += gridDim.x) {
-    const int c = L.alist[w];
-    const int inst = a.chunk_inst[c];
-    if (L.inst[inst].done) continue;
-    const bool gnn = L.inst[inst].mode == kModeGnn;  // z comes from the GNN layers
-    const V av = P::alpha(L.inst[inst]), nav = P::neg(av);
-    typename P::Acc rr, rz;
-    const int t1 = a.chunk_tile0[c + 1];
-#pragma unroll 2
-    for (int t = a.chunk_tile0[c]; t < t1; ++t) {
-      const int64_t i = (int64_t)t * kBThreads + threadIdx.x;
-      x[i] = P::fma(av, p[i], x[i]);
-      const V ri = P::fma(nav, q[i], r[i]);
-      r[i] = ri;
-      const V zi = invdiag ? P::mul(ri, invdiag[i]) : ri;
-      if (!gnn) z[i] = zi;
-      rr.add(ri, ri);
-      rz.add(ri, zi);
-    }
-    const double v[2] = {bsum<kBThreads>(rr), bsum<kBThreads>(rz)};
-    double tot[2];
-    if (chunk_finish<2>(a, c, inst, v, L, tot) && threadIdx.x == 0) {
-      esr_bcg_inst &s = L.inst[inst];
-      s.iters += 1;
-      s.rr = tot[0];
-      s.rz_jac = tot[1];
-      s.refresh = 0;
-      const double rnorm = sqrt(tot[0]);
-      if (!isnan(rnorm) && rnorm <= s.tol) {
-        s.done = 1;
-        retire(L);
-      } else if (s.maxiter >= 0 && s.iters - 1 >= s.maxiter) {
-        s.done = 2;
-        retire(L);
-      } else if (!isfinite(rnorm) || !isfinite(tot[1]) || s.rz == 0.0) {
-        s.done = 3;
-        retire(L);
-      } else if (s.mode == kModeGnn) {
-        // beta follows from the GNN output (gnn.cu); here: input scale and
-        // the stall test (no decrease of r.r over a window -> Jacobi)
-        s.sigma = s.nrows > 0 ? sqrt(tot[0] / s.nrows) : 0.0;
-        if (a.stall_window > 0 && s.iters % a.stall_window == 0) {
-          const bool clipped = 2 * (s.clips - s.clips_mark) > a.stall_window;
-          s.clips_mark = s.clips;
-          if (!(tot[0] < s.rr_mark) || clipped) {
-            s.mode = kModeJacobi;
-            s.refresh = 1;
-            s.fallbacks += 1;
-            s.gnn_iters = s.iters;
-            set_beta(s, 0.0);
-            s.rz = tot[1];
-          } else {
-            s.rr_mark = tot[0];
-          }
-        }
-      } else if (!a.poly) {  // polynomial: beta and r.z follow the sweeps
-        set_beta(s, tot[1] / s.rz);
-        s.rz = tot[1];
+  static constexpr int S = 4, K = 2;
+  static constexpr uint32_t kSweep = 2;
+  static constexpr int kStageBytes = 5 * kTileBytes;
+  struct Meta {};
+
+  const BArgs &a;
+  const V *__restrict__ invdiag;
+  V *__restrict__ x, *__restrict__ r, *__restrict__ z;
+  const V *__restrict__ p, *__restrict__ q;
+  bool wide;
+  typename P::Acc acc[2];  // r.r, r.z
+
+  static __device__ __forceinline__ V coefficient(const esr_bcg_inst &s) { return P::alpha(s); }
+  static __device__ __forceinline__ bool flag(const esr_bcg_inst &s) { return s.mode == kModeGnn; }
+  __device__ __forceinline__ Meta meta(int, int) const { return Meta{}; }
+  // stage: x, p, r, q, invdiag
+  __device__ __forceinline__ void fetch(int t, const Meta &, char *stage, int2 *, uint64_t *bar, int lane) const {
+    const int64_t i = (int64_t)t * kBThreads;
+    const int arrays = invdiag ? 5 : 4;
+    if (wide) {
+      if (lane == 0) {
+        bar_arrive_expect(bar, arrays * kTileBytes);
+        bulk_copy(stage, x + i, kTileBytes, bar);
+        bulk_copy(stage + kTileBytes, p + i, kTileBytes, bar);
+        bulk_copy(stage + 2 * kTileBytes, r + i, kTileBytes, bar);
+        bulk_copy(stage + 3 * kTileBytes, q + i, kTileBytes, bar);
+        if (invdiag) bulk_copy(stage + 4 * kTileBytes, invdiag + i, kTileBytes, bar);
       }
+    } else {
+      plain_copy(stage, x + i, kTileBytes, lane);
+      plain_copy(stage + kTileBytes, p + i, kTileBytes, lane);
+      plain_copy(stage + 2 * kTileBytes, r + i, kTileBytes, lane);
+      plain_copy(stage + 3 * kTileBytes, q + i, kTileBytes, lane);
+      if (invdiag) plain_copy(stage + 4 * kTileBytes, invdiag + i, kTileBytes, lane);
+      __syncwarp();
+      if (lane == 0) bar_arrive(bar);
     }
   }
+  __device__ __forceinline__ void compute(int t, const char *stage, int2, V av, int gnn) {
+    const int64_t i = (int64_t)t * kBThreads + threadIdx.x;
+    const V *own = (const V *)stage + threadIdx.x;
+    x[i] = P::fma(av, own[kBThreads], own[0]);
+    const V ri = P::fma(P::neg(av), own[3 * kBThreads], own[2 * kBThreads]);
+    r[i] = ri;
+    const V zi = invdiag ? P::mul(ri, own[4 * kBThreads]) : ri;
+    if (!gnn) z[i] = zi;  // (else z comes from the GNN layers)
+    acc[0].add(ri, ri);
+    acc[1].add(ri, zi);
+  }
+  BcgLayout L;
+  __device__ __forceinline__ void finish(esr_bcg_inst &s, const double (&tot)[2]) const {
+    s.iters += 1;
+    s.rr = tot[0];
+    s.rz_jac = tot[1];
+    s.refresh = 0;
+    const double rnorm = sqrt(tot[0]);
+    if (!isnan(rnorm) && rnorm <= s.tol) {
+      s.done = 1;
+      retire(L);
+    } else if (s.maxiter >= 0 && s.iters - 1 >= s.maxiter) {
+      s.done = 2;
+      retire(L);
+    } else if (!isfinite(rnorm) || !isfinite(tot[1]) || s.rz == 0.0) {
+      s.done = 3;
+      retire(L);
+    } else if (s.mode == kModeGnn) {
+      // beta follows from the GNN output (gnn.cu); here: input scale and
+      // the stall test (no decrease of r.r over a window -> Jacobi)
+      s.sigma = s.nrows > 0 ? sqrt(tot[0] / s.nrows) : 0.0;
+      if (a.stall_window > 0 && s.iters % a.stall_window == 0) {
+        const bool clipped = 2 * (s.clips - s.clips_mark) > a.stall_window;
+        s.clips_mark = s.clips;
+        if (!(tot[0] < s.rr_mark) || clipped) {
+          s.mode = kModeJacobi;
+          s.refresh = 1;
+          s.fallbacks += 1;
+          s.gnn_iters = s.iters;
+          set_beta(s, 0.0);
+          s.rz = tot[1];
+        } else {
+          s.rr_mark = tot[0];
+        }
+      }
+    } else if (!a.poly) {  // polynomial: beta and r.z follow the sweeps
+      set_beta(s, tot[1] / s.rz);
+      s.rz = tot[1];
+    }
+  }
+};
+
+template <class P>
+__global__ void __launch_bounds__(kStreamThreads, kUpdateCtas)
+bcg_update_kernel(BArgs a, const typename P::V *__restrict__ invdiag, typename P::V *__restrict__ x,
+                  typename P::V *__restrict__ r, typename P::V *__restrict__ z, const typename P::V *__restrict__ p,
+                  const typename P::V *__restrict__ q, bool wide, BcgLayout L) {
+  using OP = UpdateSweep<P>;
+  extern __shared__ __align__(128) char s_ring[];
+  __shared__ StreamShared<P, OP::S, OP::K> s_stream;
+  OP op{a, invdiag, x, r, z, p, q, wide, {}, L};
+  stream_chunks(a, L, s_ring, s_stream, op);
 }
 
 // ---- polynomial-Jacobi sweep: y_out = y_in + W (r - A y_in), persistent
@@ -536,6 +668,24 @@ int run_iterate(const esr_batch *B, void *x, void *r, void *z, void *p, void *q,
   using V = typename P::V;
   BcgLayout L = layout_of(ws, B->ninst, B->nchunks);
   const BArgs a = bargs(B);
+  // 16-byte copies where every array they read starts on 16 bytes (else 4)
+  bool wide = true;
+  for (const void *v : {(const void *)B->col, B->val, B->diag, B->invdiag, (const void *)x, (const void *)r,
+                        (const void *)z, (const void *)p, (const void *)q})
+    wide = wide && (uintptr_t)v % 16 == 0;
+  constexpr int pq_smem = PqSweep<P>::S * PqSweep<P>::kStageBytes;
+  constexpr int update_smem = UpdateSweep<P>::S * UpdateSweep<P>::kStageBytes;
+  cudaError_t e = cudaFuncSetAttribute(bcg_update_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, update_smem);
+  if constexpr (P::kFusedDirection)
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(bcg_pq_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, pq_smem);
+  if (e != cudaSuccess) return esr::cuda_check(e, "esr_bcg_iterate/smem attribute");
+  int dev = 0, sms = 0;
+  e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e != cudaSuccess) return esr::cuda_check(e, "esr_bcg_iterate/SM count");
+  // the streamed sweeps gain nothing from CTAs beyond the resident ones
+  const int pq_grid = std::min(B->grid, kPqCtas * sms), update_grid = std::min(B->grid, kUpdateCtas * sms);
   bcg_compact_kernel<<<1, 1024, 0, s>>>(a, L);
   const int d = B->poly_degree;
   V *const tmp0 = (V *)B->poly_tmp, *const tmp1 = tmp0 ? tmp0 + B->n : nullptr;
@@ -556,13 +706,13 @@ int run_iterate(const esr_batch *B, void *x, void *r, void *z, void *p, void *q,
         bcg_pupdate_kernel<P><<<B->grid, kBThreads, 0, s>>>(a, (const V *)z, (V *)p, L);
     }
     if constexpr (P::kFusedDirection)
-      bcg_pq_kernel<P><<<B->grid, kBThreads, 0, s>>>(a, (const V *)B->val, (const V *)B->diag, (const V *)z, (V *)p,
-                                                     (V *)q, L);
+      bcg_pq_kernel<P><<<pq_grid, kStreamThreads, pq_smem, s>>>(a, (const V *)B->val, (const V *)B->diag,
+                                                                (const V *)z, (V *)p, (V *)q, wide, L);
     else
       bcg_spmv_kernel<P><<<B->grid, kBThreads, 0, s>>>(a, (const V *)B->val, (const V *)B->diag, (const V *)p,
                                                        (V *)q, L);
-    bcg_update_kernel<P><<<B->grid, kBThreads, 0, s>>>(a, (const V *)B->invdiag, (V *)x, (V *)r, (V *)z,
-                                                       (const V *)p, (const V *)q, L);
+    bcg_update_kernel<P><<<update_grid, kStreamThreads, update_smem, s>>>(
+        a, (const V *)B->invdiag, (V *)x, (V *)r, (V *)z, (const V *)p, (const V *)q, wide, L);
     if (B->gnn) {
       const int st = esr::gnn_layers(B, r, q, z, ws, s);
       if (st) return st;
@@ -688,6 +838,8 @@ void destroy_graph(BcgGraph *G) {
 }
 
 }  // namespace
+
+ESR_DEFINE_STATUS_READER(esr_status_bcg)
 
 extern "C" int esr_bcg_graph_create(const esr_batch *B, const double *b64, const void *b, void *x, void *r, void *z,
                                     void *p, void *q, double *x64, double *r64, double rtol, double atol,

@@ -16,6 +16,7 @@ namespace {
 
 constexpr int kBThreads = 256;  // rows per tile: one row per thread per tile
 constexpr int kBSums = 3;       // partial arrays
+constexpr int kCounterStride = 32;  // words: an instance's tickets have a line of their own
 
 struct BcgHead {
   int32_t active;  // instances with done == 0
@@ -29,6 +30,8 @@ struct BcgLayout {
   esr_bcg_inst *inst;
   unsigned int *counter;  // [ninst] arrival tickets
   int32_t *alist;         // [nchunks] active chunk list
+  int4 *heads;            // [nchunks] of each entry: the chunk, its instance, its tiles [z, w)
+  ulonglong2 *mail;       // [2][nchunks] chunk sums of the streamed sweeps, tagged (bcg_stream.cuh)
   double *partial;        // [kBSums][nblocks] (chunk or tile partials)
 };
 
@@ -42,16 +45,21 @@ BcgLayout layout_of(void *ws, int32_t ninst, int32_t nchunks) {
   L.inst = (esr_bcg_inst *)p;
   p += round256(ninst * (int64_t)sizeof(esr_bcg_inst));
   L.counter = (unsigned int *)p;
-  p += round256(ninst * (int64_t)sizeof(unsigned int));
+  p += round256(ninst * (int64_t)(kCounterStride * sizeof(unsigned int)));
   L.alist = (int32_t *)p;
   p += round256(nchunks * (int64_t)sizeof(int32_t));
+  L.heads = (int4 *)p;
+  p += round256(nchunks * (int64_t)sizeof(int4));
+  L.mail = (ulonglong2 *)p;
+  p += 2 * round256(nchunks * (int64_t)sizeof(ulonglong2));
   L.partial = (double *)p;
   return L;
 }
 
 int64_t workspace_bytes(int32_t ninst, int32_t nblocks, int32_t nchunks) {
   return round256(sizeof(BcgHead)) + round256(ninst * (int64_t)sizeof(esr_bcg_inst)) +
-         round256(ninst * (int64_t)sizeof(unsigned int)) + round256(nchunks * (int64_t)sizeof(int32_t)) +
+         round256(ninst * (int64_t)(kCounterStride * sizeof(unsigned int))) + round256(nchunks * (int64_t)sizeof(int32_t)) +
+         round256(nchunks * (int64_t)sizeof(int4)) + 2 * round256(nchunks * (int64_t)sizeof(ulonglong2)) +
          kBSums * (int64_t)nblocks * (int64_t)sizeof(double);
 }
 
@@ -301,7 +309,7 @@ template <int K>
 __device__ __forceinline__ bool tile_finish(const BArgs &a, int inst, const double (&v)[K], BcgLayout L,
                                             double (&tot)[K]) {
   const int b0 = a.inst_block0[inst], b1 = a.inst_block0[inst + 1];
-  return inst_finish<K>(v, blockIdx.x, b0, b1, b1 - b0, a.nblocks, L.partial, L.counter + inst, tot);
+  return inst_finish<K>(v, blockIdx.x, b0, b1, b1 - b0, a.nblocks, L.partial, L.counter + inst * (int64_t)kCounterStride, tot);
 }
 
 // chunk finish (persistent kernels)
@@ -309,7 +317,7 @@ template <int K, int THREADS = kBThreads>
 __device__ __forceinline__ bool chunk_finish(const BArgs &a, int chunk, int inst, const double (&v)[K],
                                              BcgLayout L, double (&tot)[K]) {
   const int c0 = a.inst_chunk0[inst], c1 = a.inst_chunk0[inst + 1];
-  return inst_finish<K, THREADS>(v, chunk, c0, c1, c1 - c0, a.nblocks, L.partial, L.counter + inst, tot);
+  return inst_finish<K, THREADS>(v, chunk, c0, c1, c1 - c0, a.nblocks, L.partial, L.counter + inst * (int64_t)kCounterStride, tot);
 }
 
 // Flexible-CG (GNN preconditioner) modes of an instance

@@ -10,6 +10,7 @@ int esr_status_gather_reduce(int *bits, int clear, cudaStream_t s);
 int esr_status_swe(int *bits, int clear, cudaStream_t s);
 int esr_status_cg(int *bits, int clear, cudaStream_t s);
 int esr_status_gnn(int *bits, int clear, cudaStream_t s);
+int esr_status_bcg(int *bits, int clear, cudaStream_t s);
 int esr_status_pcg_solo(int *bits, int clear, cudaStream_t s);
 int esr_status_gmres(int *bits, int clear, cudaStream_t s);
 int esr_status_mesh_gpu(int *bits, int clear, cudaStream_t s);
@@ -30,6 +31,7 @@ extern "C" int esr_device_status(int *status_out, int clear, void *stream) {
   if ((st = esr_status_swe(&bits, clear, s))) return st;
   if ((st = esr_status_cg(&bits, clear, s))) return st;
   if ((st = esr_status_gnn(&bits, clear, s))) return st;
+  if ((st = esr_status_bcg(&bits, clear, s))) return st;
   if ((st = esr_status_pcg_solo(&bits, clear, s))) return st;
   if ((st = esr_status_gmres(&bits, clear, s))) return st;
   if ((st = esr_status_mesh_gpu(&bits, clear, s))) return st;
