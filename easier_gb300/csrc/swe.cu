@@ -123,6 +123,25 @@ struct Acc3 {
   T Bu, Bv;      // scatter_b(...) over wall faces
 };
 
+// The flux terms of one interior face in the reference's operations and order.
+template <typename T>
+__device__ __forceinline__ void exact_face(T oh, T ou, T ov, T nh, T nu, T nv, T a, T fx, T fy, T &Fh, T &Fu, T &Fv) {
+  using A = Ar<T, true>;
+  const T om = A::sub(T(1), a);
+  const T hf = A::imadd(om, nh, A::imul(a, oh));   // (1 - alpha)*h[src] + alpha*h[dst]
+  const T uhf = A::imadd(om, nu, A::imul(a, ou));
+  const T vhf = A::imadd(om, nv, A::imul(a, ov));
+  const auto by_hf = A::divisor(hf);
+  const T uf = A::quot(uhf, by_hf);
+  const T vf = A::quot(vhf, by_hf);
+  const T hfs = A::imul(A::half(hf), hf);        // 0.5 * h_f * h_f
+  const T uhsx = A::mul(uhf, fx);                // uh_f * sx
+  const T vhsy = A::mul(vhf, fy);                // vh_f * sy
+  Fh = A::add(uhsx, vhsy);
+  Fu = A::madd(A::imadd(uf, uhf, hfs), fx, A::imul(uf, vhsy));
+  Fv = A::imadd(vf, uhsx, A::mul(A::imadd(vf, vhf, hfs), fy));
+}
+
 // One interior face of a cell: flux terms of swe_main.py:87-117 added to the
 // cell's sums.  own/nb = (h, uh, vh) of the destination (this cell) and the
 // source (neighbour).
@@ -148,19 +167,8 @@ __device__ __forceinline__ void add_face(Acc3<T> &s, T oh, T ou, T ov, T nh, T n
     s.Su = A::madd(uhf, Fi, A::madd(hfs, fx, s.Su));
     s.Sv = A::madd(vhf, Fi, A::madd(hfs, fy, s.Sv));
   } else {
-    const T om = A::sub(T(1), a);
-    const T hf = A::imadd(om, nh, A::imul(a, oh));   // (1 - alpha)*h[src] + alpha*h[dst]
-    const T uhf = A::imadd(om, nu, A::imul(a, ou));
-    const T vhf = A::imadd(om, nv, A::imul(a, ov));
-    const auto by_hf = A::divisor(hf);
-    const T uf = A::quot(uhf, by_hf);
-    const T vf = A::quot(vhf, by_hf);
-    const T hfs = A::imul(A::half(hf), hf);        // 0.5 * h_f * h_f
-    const T uhsx = A::mul(uhf, fx);                // uh_f * sx
-    const T vhsy = A::mul(vhf, fy);                // vh_f * sy
-    const T Fh = A::add(uhsx, vhsy);
-    const T Fu = A::madd(A::imadd(uf, uhf, hfs), fx, A::imul(uf, vhsy));
-    const T Fv = A::imadd(vf, uhsx, A::mul(A::imadd(vf, vhf, hfs), fy));
+    T Fh, Fu, Fv;
+    exact_face<T>(oh, ou, ov, nh, nu, nv, a, fx, fy, Fh, Fu, Fv);
     if constexpr (FIRST) {
       s.Sh = A::from_zero(Fh);
       s.Su = A::from_zero(Fu);
@@ -327,6 +335,92 @@ swe_stage_kernel(int64_t nc, SlotsG<T> g, const T *__restrict__ sin, const T *s0
   store4(sout + 4 * i, out);
 }
 
+// The same stage with a lane a face, for meshes too small to fill the chip with
+// a thread a cell: lane k of a cell's W lanes takes face k, then component k of
+// the sums, the division by the area and the update.  Every value comes from
+// the same operations in the same order.
+constexpr int kFaceThreads = 128;
+
+template <int W>
+constexpr int kFaceCells = kFaceThreads / 32 * (32 / W);  // cells a CTA
+
+template <int W, int STAGE>
+__global__ void __launch_bounds__(kFaceThreads, 8)
+swe_face_kernel(int64_t nc, SlotsG<double> g, const double *sin, const double *s0, double *acc, double *sout,
+                double c) {
+  using A = Ar<double, true>;
+  __shared__ double s_face[kFaceThreads / 32][32][3];
+  const int warp = threadIdx.x >> 5, cell = (threadIdx.x & 31) / W, k = (threadIdx.x & 31) - cell * W;
+  const int64_t i = (int64_t)blockIdx.x * kFaceCells<W> + warp * (32 / W) + cell;
+  const bool in = cell < 32 / W && i < nc;
+  int32_t j = -2;
+  double fx = 0.0, fy = 0.0, a = 0.0, area = 1.0;
+  if (in) {
+    const int64_t slot = k * nc + i;
+    j = __ldg(g.nbr + slot);
+    fx = __ldg(g.sx + slot);
+    fy = __ldg(g.sy + slot);
+    a = __ldg(g.alpha + slot);
+    area = __ldg(g.area + i);
+  }
+  const auto by_area = A::divisor(area);
+  // (all that depends on the mesh alone comes while the stage before runs)
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (j >= 0 && (int64_t)j >= nc) {  // corrupt slot: flag it, never read out of bounds
+    esr::raise_status(ESR_DEV_IDX_RANGE);
+    j = -2;
+  }
+  double *mine = s_face[warp][threadIdx.x & 31];
+  if (in) {
+    const Vec4<double> own = load4(sin + 4 * i);
+    if (j >= 0) {
+      const Vec4<double> nb = load4(sin + 4 * (int64_t)j);
+      exact_face<double>(own.x, own.y, own.z, nb.x, nb.y, nb.z, a, fx, fy, mine[0], mine[1], mine[2]);
+    } else if (j == -1) {
+      const double gb = A::mul(0.5, A::mul(own.x, own.x));
+      mine[1] = A::mul(gb, fx);
+      mine[2] = A::mul(gb, fy);
+    }
+  }
+  const unsigned faces = __ballot_sync(0xffffffffu, j >= 0) >> (cell * W);
+  const unsigned walls = (__ballot_sync(0xffffffffu, j == -1) >> (cell * W)) & ((1 << W) - 1);
+  __syncwarp();
+  if (!in) return;
+  const int64_t at = 4 * i + k;
+  if (k == 3) {  // (the state's fourth word; there are four lanes)
+    sout[at] = STAGE < 4 ? 0.0 : s0[at];
+    if (STAGE == 1) acc[at] = 0.0;
+    return;
+  }
+  if (W == 3 && k == 0) {
+    sout[at + 3] = STAGE < 4 ? 0.0 : s0[at + 3];
+    if (STAGE == 1) acc[at + 3] = 0.0;
+  }
+  const double base = s0[at], prev = STAGE > 1 ? acc[at] : 0.0;
+  const double(*terms)[3] = s_face[warp] + cell * W;
+  double S = 0.0;
+#pragma unroll
+  for (int f = 0; f < W; ++f)
+    if (faces >> f & 1) S = A::add(S, terms[f][k]);
+  if (k > 0) {
+    double B = 0.0;
+    if (walls) {
+#pragma unroll
+      for (int f = 0; f < W; ++f)
+        if (walls >> f & 1) B = A::add(terms[f][k], B);
+    }
+    S = A::add(S, B);
+  }
+  const double d = A::quot(A::neg(S), by_area);
+  if (STAGE < 4) {
+    acc[at] = STAGE == 1 ? d : A::add(prev, d);
+    sout[at] = A::imadd(c, d, base);
+  } else {
+    sout[at] = A::madd(c, A::add(prev, d), base);
+  }
+}
+
 template <typename T, int W, bool EXACT>
 __global__ void __launch_bounds__(kSweThreads)
 swe_delta_kernel(int64_t nc, SlotsG<T> g, const T *__restrict__ s, T *__restrict__ dout) {
@@ -358,9 +452,50 @@ SlotsG<T> slots_of(const esr_swe_mesh *m) {
 // five SMs with twice the others' work).
 int stage_threads(int64_t nc) { return nc < (int64_t)152 * 16 * kStageThreads ? 64 : kStageThreads; }
 
+// Up to 100,000 cells a thread a cell leaves the chip waiting on a few warps'
+// serial arithmetic; a lane a face has three times the warps, a third of the
+// chain, and loads the mesh while the stage before still runs.  A step, from
+// rest / in flow: 10,000 cells 54.7 / 47.6 -> 30.9 / 31.1 us, 22,500 cells
+// 60.5 / 50.9 -> 37.6 / 33.9, 40,000 cells 66.3 / 55.2 -> 54.2 / 47.9, 80,000
+// cells 85.1 / 69.2 -> 78.0 / 66.6.  At 160,000 cells the chip is full either
+// way and the idle lanes cost: 131.4 / 110.2 against 131.0 / 113.8.  (Four
+// lanes a cell in place of three: 60.0 at 40,000.  Early launch of the
+// thread-a-cell kernel: 60.8 there, but 92.1 against 85.1 at 80,000.)
+bool face_stages(int64_t nc) { return nc <= 100000; }
+
+template <int W>
+int run_face_steps(const esr_swe_mesh *m, double dt, double *state, int64_t steps, double *ws, cudaStream_t st) {
+  const int64_t nc = m->nc;
+  double *S1 = ws, *S2 = ws + 4 * nc, *A = ws + 8 * nc;
+  const SlotsG<double> g = slots_of<double>(m);
+  const double c1 = 0.5 * dt, c4 = dt / 6;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)((nc + kFaceCells<W> - 1) / kFaceCells<W>));
+  cfg.blockDim = dim3(kFaceThreads);
+  cfg.stream = st;
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  const double *in = state;
+  cudaError_t e = cudaSuccess;
+  for (int64_t s = 0; s < steps && e == cudaSuccess; ++s) {
+    cfg.numAttrs = s > 0 ? 1 : 0;  // (the first follows launches that are not ours)
+    e = cudaLaunchKernelEx(&cfg, swe_face_kernel<W, 1>, nc, g, in, in, A, S1, c1);
+    cfg.numAttrs = 1;
+    if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, swe_face_kernel<W, 2>, nc, g, (const double *)S1, in, A, S2, c1);
+    if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, swe_face_kernel<W, 3>, nc, g, (const double *)S2, in, A, S1, dt);
+    if (e == cudaSuccess)
+      e = cudaLaunchKernelEx(&cfg, swe_face_kernel<W, 4>, nc, g, (const double *)S1, in, A, state, c4);
+  }
+  return e == cudaSuccess ? ESR_OK : esr::cuda_check(e, "esr_swe_step");
+}
+
 template <typename T, int W, bool EXACT>
 int run_steps(const esr_swe_mesh *m, double dt, T *state, int64_t steps, T *ws, cudaStream_t st) {
   const int64_t nc = m->nc;
+  if constexpr (EXACT && std::is_same<T, double>::value)
+    if (face_stages(nc)) return run_face_steps<W>(m, dt, state, steps, ws, st);
   const int threads = stage_threads(nc);
   const int grid = (int)((nc + threads - 1) / threads);
   T *S1 = ws;
