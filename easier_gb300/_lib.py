@@ -12,6 +12,8 @@ import threading
 from ctypes import POINTER, Structure, c_double, c_int, c_int32, c_int64, c_void_p, c_char_p
 from pathlib import Path
 
+import torch
+
 from .utils import EasierJitException
 
 F32, F64, I32, I64 = 0, 1, 2, 3
@@ -208,7 +210,10 @@ def check(status: int, what: str = "") -> None:
 
 
 def call(name: str, *args) -> None:
-    check(getattr(lib(), name)(*args), name)
+    # (on the path of every small op: one attribute of the loaded library)
+    status = getattr(_LIB or lib(), name)(*args)
+    if status:
+        check(status, name)
 
 
 def ptr(t) -> int:
@@ -221,13 +226,22 @@ def ptr(t) -> int:
 
 
 def stream_handle(device=None) -> int:
-    import torch
-    return torch.cuda.current_stream(device).cuda_stream
+    """torch's current stream on ``device`` (an index, a device or its name,
+    None for the current one) as a raw handle, without a Stream object."""
+    if device.__class__ is not int:
+        if device is not None and device.__class__ is not torch.device:
+            device = torch.device(device)
+        if device is not None and device.type != "cuda":
+            raise ValueError(f"expected a CUDA device, not {device}")
+        device = torch.cuda.current_device() if device is None or device.index is None else device.index
+    return torch._C._cuda_getCurrentRawStream(device)
+
+
+_DTYPE_CODES = {torch.float32: F32, torch.float64: F64, torch.int32: I32, torch.int64: I64}
 
 
 def dtype_code(dtype) -> int:
-    import torch
-    m = {torch.float32: F32, torch.float64: F64, torch.int32: I32, torch.int64: I64}
-    if dtype not in m:
+    code = _DTYPE_CODES.get(dtype)
+    if code is None:
         raise NotImplementedError(f"dtype {dtype} is not supported by the GB300 path")
-    return m[dtype]
+    return code

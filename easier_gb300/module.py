@@ -16,6 +16,7 @@ from typing import Dict, List, Literal, Optional, Sequence, Tuple, Union
 import torch
 from torch import nn
 
+from . import ops
 from .data_loader import (ATTRIBUTE_PLACEHOLDER, ArangeTensorLoader, DataLoaderBase, FulledTensorLoader,
                           H5DataLoader, InMemoryTensorLoader)
 from .utils import EasierJitException
@@ -131,7 +132,6 @@ class Selector(nn.Module):
     def forward(self, tensor: torch.Tensor) -> torch.Tensor:
         if self.easier_index_status != "rewritten":
             raise RuntimeError("Selector.idx not ready, run compile() first")
-        from . import ops
         return ops.select(self, tensor)
 
     def to(self, device: Union[str, torch.device]):
@@ -178,7 +178,6 @@ class Reducer(nn.Module):
             raise ValueError(
                 f"{out.shape[0]} the length of the first dimension of `out`"
                 f" and {self.n} the specified `Reducer.n` do not match")
-        from . import ops
         return ops.reduce(self, tensor, out)
 
     def to(self, device: Union[str, torch.device]):
@@ -328,12 +327,10 @@ class Module(nn.Module):
 # ---------------------------------------------------------- aggregators
 def sum(tensor: torch.Tensor) -> torch.Tensor:
     """``torch.sum(t, dim=0, keepdim=True)`` (module.py:829-837)."""
-    from . import ops
     return ops.aggregate(tensor, "sum")
 
 
 def prod(tensor: torch.Tensor) -> torch.Tensor:
-    from . import ops
     return ops.aggregate(tensor, "prod")
 
 
@@ -341,17 +338,14 @@ def norm(tensor: torch.Tensor, p: Union[int, str] = 2) -> torch.Tensor:
     """``torch.norm(t, p, dim=0, keepdim=True)``; p = 2 only."""
     if p not in (2, "fro"):
         raise NotImplementedError("easier_gb300 implements the 2-norm aggregator only")
-    from . import ops
     return ops.aggregate(tensor, "norm")
 
 
 def max(tensor: torch.Tensor) -> torch.Tensor:
-    from . import ops
     return ops.aggregate(tensor, "max")
 
 
 def min(tensor: torch.Tensor) -> torch.Tensor:
-    from . import ops
     return ops.aggregate(tensor, "min")
 
 

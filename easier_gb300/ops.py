@@ -6,6 +6,7 @@ current stream.  Non-CUDA tensors raise: there is no CPU path.
 """
 from __future__ import annotations
 
+from math import prod
 from typing import Optional
 
 import torch
@@ -16,7 +17,7 @@ from .utils import EasierJitException
 
 
 def _require_cuda(t: torch.Tensor, what: str) -> None:
-    if not isinstance(t, torch.Tensor) or t.device.type != "cuda":
+    if not (isinstance(t, torch.Tensor) and t.is_cuda):
         raise EasierJitException(f"{what}: easier_gb300 runs on CUDA tensors only (got {getattr(t, 'device', type(t))})")
 
 
@@ -24,16 +25,17 @@ def select(sel, tensor: torch.Tensor) -> torch.Tensor:
     """Selector.forward: tensor[idx] (easier/core/module.py:364-371)."""
     _require_cuda(tensor, "Selector")
     idx = sel._idx32
-    if idx.device != tensor.device:
+    index = tensor.get_device()
+    if idx.get_device() != index:
         raise EasierJitException("Selector input is on a different device than its index")
-    if sel._idx_max >= tensor.shape[0]:
-        raise IndexError(f"index {sel._idx_max} is out of bounds for dimension 0 with size {tensor.shape[0]}")
+    shape = tensor.shape
+    if sel._idx_max >= shape[0]:
+        raise IndexError(f"index {sel._idx_max} is out of bounds for dimension 0 with size {shape[0]}")
     src = tensor.contiguous()
     m = idx.shape[0]
-    out = torch.empty((m,) + tuple(src.shape[1:]), dtype=src.dtype, device=src.device)
-    row_bytes = src.element_size() * int(torch.Size(src.shape[1:]).numel())
-    _lib.call("esr_gather", _lib.ptr(src), src.shape[0], row_bytes, _lib.ptr(idx), m, _lib.ptr(out),
-              _lib.stream_handle(src.device))
+    out = torch.empty((m, *shape[1:]), dtype=src.dtype, device=src.device)
+    _lib.call("esr_gather", src.data_ptr(), shape[0], src.element_size() * prod(shape[1:]), idx.data_ptr(), m,
+              out.data_ptr(), _lib.stream_handle(index))
     return out
 
 
@@ -51,22 +53,22 @@ def reduce(red, tensor: torch.Tensor, out: Optional[torch.Tensor] = None) -> tor
     _require_cuda(tensor, "Reducer")
     op = _lib.REDUCE_OPS[red.reduce]
     if out is None:
-        out = torch.empty((red.n,) + tuple(tensor.shape[1:]), dtype=tensor.dtype, device=tensor.device)
+        out = torch.empty((red.n, *tensor.shape[1:]), dtype=tensor.dtype, device=tensor.device)
         op |= _lib.REDUCE_FILL
     else:
         _require_cuda(out, "Reducer out")
     if tensor.dtype != out.dtype:
         raise RuntimeError(f"scatter_reduce(): Expected self.dtype to be equal to src.dtype ({out.dtype} vs {tensor.dtype})")
     m = red._perm32.shape[0]
-    if tensor.shape[0] < m or tuple(tensor.shape[1:]) != tuple(out.shape[1:]):
+    row = tensor.shape[1:]
+    if tensor.shape[0] < m or row != out.shape[1:]:
         raise RuntimeError(
             f"Reducer: input of shape {tuple(tensor.shape)} does not match idx length {m} and"
             f" out shape {tuple(out.shape)}")
     src = tensor.contiguous()
     dst = out if out.is_contiguous() else out.contiguous()
-    cols = int(torch.Size(src.shape[1:]).numel())
-    _lib.call("esr_segreduce", _lib.dtype_code(src.dtype), op, _lib.ptr(src), cols, _lib.ptr(red._rowptr32),
-              _perm_ptr(red), red.n, _lib.ptr(dst), _lib.stream_handle(src.device))
+    _lib.call("esr_segreduce", _lib.dtype_code(src.dtype), op, src.data_ptr(), prod(row), red._rowptr32.data_ptr(),
+              _perm_ptr(red), red.n, dst.data_ptr(), _lib.stream_handle(src.get_device()))
     if dst is not out:
         out.copy_(dst)
     return out
@@ -94,22 +96,40 @@ def linsys_apply(A, x: torch.Tensor) -> Optional[torch.Tensor]:
     bitwise the five-step form), or None where the five steps could do
     anything else: other shapes and dtypes (broadcasts, promotion), gradients,
     hooks, subclasses, an index out of range."""
-    from .module import Reducer, Selector, Tensor
     sel, red, Ae, Av = A.selector, A.reducer, A.Ae, A.Av
-    if type(sel) is not Selector or type(red) is not Reducer or red.reduce != "sum"             or sel.easier_index_status != "rewritten" or red.easier_index_status != "rewritten"             or not _plain_call(sel) or not _plain_call(red) or _observed():
+    plain, Selector, Reducer = _linsys_types or _set_linsys_types()
+    if (type(sel) is not Selector or type(red) is not Reducer or red.reduce != "sum"
+            or sel.easier_index_status != "rewritten" or red.easier_index_status != "rewritten"
+            or not _plain_call(sel) or not _plain_call(red) or _observed()):
         return None
-    for t in (x, Ae, Av):
-        if type(t) not in (torch.Tensor, torch.nn.Parameter, Tensor) or t.dim() != 1 or t.dtype != x.dtype                 or t.device != x.device or (t.requires_grad and torch.is_grad_enabled()):
+    if type(x) not in plain or x.dim() != 1 or not x.is_cuda or x.layout is not torch.strided:
+        return None
+    dtype, index, grads = x.dtype, x.get_device(), torch.is_grad_enabled()
+    if (dtype is not torch.float32 and dtype is not torch.float64) or (grads and x.requires_grad):
+        return None
+    n, m, col = red.n, red._perm32.shape[0], sel._idx32
+    for t, length in ((Ae, m), (Av, n)):
+        if (type(t) not in plain or t.dim() != 1 or t.dtype is not dtype or t.get_device() != index
+                or (grads and t.requires_grad) or t.shape[0] != length or not t.is_contiguous()):
             return None
-    n, m = red.n, red._perm32.shape[0]
-    if x.dtype not in (torch.float32, torch.float64) or x.device.type != "cuda" or x.layout is not torch.strided             or x.shape[0] != n or Av.shape[0] != n or Ae.shape[0] != m or sel._idx32.shape[0] != m             or sel._idx_max >= n or sel._idx32.device != x.device or red._perm32.device != x.device             or not Ae.is_contiguous() or not Av.is_contiguous():
+    if (x.shape[0] != n or col.shape[0] != m or sel._idx_max >= n or col.get_device() != index
+            or red._perm32.get_device() != index):
         return None
     x = x.contiguous()
     y = torch.empty_like(x, requires_grad=False)
-    _lib.call("esr_linsys_apply", _lib.dtype_code(x.dtype), _lib.ptr(x), _lib.ptr(Ae), _lib.ptr(Av),
-              _lib.ptr(sel._idx32), _lib.ptr(red._rowptr32), _perm_ptr(red), n, _lib.ptr(y),
-              _lib.stream_handle(x.device))
+    _lib.call("esr_linsys_apply", _lib.dtype_code(dtype), x.data_ptr(), Ae.data_ptr(), Av.data_ptr(), col.data_ptr(),
+              red._rowptr32.data_ptr(), _perm_ptr(red), n, y.data_ptr(), _lib.stream_handle(index))
     return y
+
+
+_linsys_types = None  # (module.py imports this file)
+
+
+def _set_linsys_types():
+    global _linsys_types
+    from .module import Reducer, Selector, Tensor
+    _linsys_types = ((torch.Tensor, torch.nn.Parameter, Tensor), Selector, Reducer)
+    return _linsys_types
 
 
 _AGG = {"sum": _lib.AGG_SUM, "prod": _lib.AGG_PROD, "norm": _lib.AGG_NORM, "max": _lib.AGG_MAX, "min": _lib.AGG_MIN}
@@ -125,12 +145,13 @@ def aggregate(tensor: torch.Tensor, kind: str) -> torch.Tensor:
         raise IndexError(f"{kind}(): Expected reduction dim 0 to have non-zero size.")
     src = tensor.contiguous()
     n = src.shape[0]
-    cols = int(torch.Size(src.shape[1:]).numel())
-    out = torch.empty((1,) + tuple(src.shape[1:]), dtype=src.dtype, device=src.device)
+    cols = prod(src.shape[1:])
+    device = src.device
+    out = torch.empty((1, *src.shape[1:]), dtype=src.dtype, device=device)
     nbytes = _lib.lib().esr_aggregate_workspace_bytes(n, cols)
-    ws = torch.empty(max(int(nbytes), 16), dtype=torch.uint8, device=src.device)
-    _lib.call("esr_aggregate", _lib.dtype_code(src.dtype), _AGG[kind], _lib.ptr(src), n, cols, _lib.ptr(out),
-              _lib.ptr(ws), _lib.stream_handle(src.device))
+    ws = torch.empty(max(int(nbytes), 16), dtype=torch.uint8, device=device)
+    _lib.call("esr_aggregate", _lib.dtype_code(src.dtype), _AGG[kind], src.data_ptr(), n, cols, out.data_ptr(),
+              ws.data_ptr(), _lib.stream_handle(device))
     return out
 
 

@@ -50,6 +50,7 @@ WALL = ("bsx", "bsy")
 SELECTORS = ("gather_src", "gather_dst", "gather_b")
 REDUCERS = ("scatter", "scatter_b")
 STATE = ("h", "uh", "vh")
+_GEOMETRY = EDGE + WALL + ("area",)
 
 TILE_CELLS = 4096       # tile size cap (kernel limit: 4096 own cells)
 TILE_MIN_CELLS = 256
@@ -409,8 +410,9 @@ class SweEngine:
         self._fill_geometry()
 
     def _versions(self):
+        # (before every step: no tensor objects and no generator for it)
         t = self.b["tensors"]
-        return tuple((t[k].data.data_ptr(), t[k]._version) for k in EDGE + WALL + ("area",))
+        return [(v.data_ptr(), v._version) for v in [t[k] for k in _GEOMETRY]]
 
     @property
     def state(self) -> torch.Tensor:
@@ -445,7 +447,8 @@ class SweEngine:
         if self._versions() != self._geom_versions:
             self._fill_geometry()
         t = self.b["tensors"]
-        if tuple(t[k].data.data_ptr() for k in STATE) != self._state_ptrs:
+        h, uh, vh = STATE
+        if (t[h].data_ptr(), t[uh].data_ptr(), t[vh].data_ptr()) != self._state_ptrs:
             raise RuntimeError("the shallow-water state tensors were replaced after compile(); write into them in place")
 
     def step(self, steps: int = 1) -> None:
