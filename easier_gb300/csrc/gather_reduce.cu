@@ -10,6 +10,7 @@
 
 #include "esr_internal.h"
 #include "reduce_util.cuh"
+#include "soft64.cuh"
 
 namespace {
 
@@ -207,7 +208,8 @@ __device__ __forceinline__ int32_t warp_most(int32_t v) { return __reduce_max_sy
 // row bounds -> perm -> value, so a thread requests R rows' bounds, then up to
 // U positions of each, then their values, before it adds them in order;
 // longer segments go on U entries at a time.  Load::entry(k) gives an entry's
-// position, fetch() loads what lies there, value() turns that into the terms.
+// position, fetch() loads what lies there, follow() what that points to, value()
+// turns it into the terms.
 // Rows without entries reach the store with `none` set.  (Staging the entries
 // through shared memory so that perm loads coalesce was slower: 131 us against
 // 52 for a plain loop per (row, column) at 1.96 M rows of 3 entries x 3 FP32
@@ -235,6 +237,11 @@ __device__ __forceinline__ void seg_rows(const Load &load, const Store &store, c
     for (int u = 0; u < U; ++u)
       if (u < e[q] - b[q]) load.fetch(src[q][u], col[q], h[q][u]);
 #pragma unroll
+  for (int q = 0; q < R; ++q)
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (u < e[q] - b[q]) load.follow(h[q][u]);
+#pragma unroll
   for (int q = 0; q < R; ++q) {
     T acc[D];
 #pragma unroll
@@ -258,6 +265,9 @@ __device__ __forceinline__ void seg_rows(const Load &load, const Store &store, c
 #pragma unroll
       for (int u = 0; u < U; ++u)
         if (u < left) load.fetch(src[q][u], col[q], h[q][u]);
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (u < left) load.follow(h[q][u]);
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         if (u >= most - done) break;
@@ -293,6 +303,7 @@ struct SegLoad {
 #pragma unroll
     for (int c = 0; c < D; ++c) h.v[c] = __ldg(p + c);
   }
+  __device__ __forceinline__ void follow(Held &) const {}
   __device__ __forceinline__ void value(const Held &h, T (&v)[D]) const {
 #pragma unroll
     for (int c = 0; c < D; ++c) v[c] = h.v[c];
@@ -400,14 +411,20 @@ int launch_segreduce(int op, const void *t, int64_t cols, const int32_t *rowptr,
 // y = reducer(selector(x) * Ae) + x * Av straight from the Selector's index
 // and the Reducer's CSR, one pass instead of five through memory, with the
 // same rounded operations in the same order (bitwise the five).  One thread
-// a row, eight entries' loads in flight; bound by the FP64 pipe in FP64 (two
-// operations an entry and two a row: 34 us of 84 before for the 998,001-row P1
-// grid, FP64 pipe 68%), by HBM in FP32.
+// a row, four entries' loads in flight, all of x's before the first product
+// (the sum's branches hold loads back); bound in FP64 by latency and the FP64
+// pipe together (two operations an entry, one a row: 75% busy), by HBM in FP32.
+// 998,001-row P1 grid, FP64: 84 us as five steps; 35 with eight entries and x
+// loaded product by product; 31 so.  The row's own product runs on the integer
+// pipe; the entries' there too: 33.  Two rows a thread: 39.
+__device__ __forceinline__ float linsys_product(float a, float b) { return ops<float>::mul(a, b); }
+__device__ __forceinline__ double linsys_product(double a, double b) { return soft64::product(a, b); }
+
 template <typename T>
 struct LinsysLoad {
   struct Held {
     int32_t col;
-    T ae;
+    T ae, x;
   };
   const T *x, *ae;
   const int32_t *col, *perm;
@@ -416,7 +433,10 @@ struct LinsysLoad {
     h.col = __ldg(col + src);
     h.ae = __ldg(ae + src);
   }
-  __device__ __forceinline__ void value(const Held &h, T (&v)[1]) const { v[0] = ops<T>::mul(__ldg(x + h.col), h.ae); }
+  __device__ __forceinline__ void follow(Held &h) const { h.x = __ldg(x + h.col); }
+  __device__ __forceinline__ void value(const Held &h, T (&v)[1]) const {
+    v[0] = ops<T>::mul(h.x, h.ae);
+  }
 };
 
 template <typename T>
@@ -424,7 +444,7 @@ struct LinsysStore {
   const T *x, *av;
   T *y;
   __device__ __forceinline__ void operator()(int64_t i, int64_t, const T (&acc)[1], bool) const {
-    y[i] = ops<T>::add(acc[0], ops<T>::mul(__ldg(x + i), __ldg(av + i)));
+    y[i] = ops<T>::add(acc[0], linsys_product(__ldg(x + i), __ldg(av + i)));
   }
 };
 
@@ -436,7 +456,7 @@ linsys_kernel(const T *__restrict__ x, const T *__restrict__ ae, const T *__rest
   const int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x;
   const int64_t row[1] = {i}, none[1] = {0};
   const bool mine[1] = {i < n};
-  seg_rows<T, ESR_REDUCE_SUM, 1, 8, 1>(LinsysLoad<T>{x, ae, col, perm}, LinsysStore<T>{x, av, y}, rowptr, row, none,
+  seg_rows<T, ESR_REDUCE_SUM, 1, 4, 1>(LinsysLoad<T>{x, ae, col, perm}, LinsysStore<T>{x, av, y}, rowptr, row, none,
                                        mine);
 }
 
