@@ -497,7 +497,7 @@ class BatchedPCG:
             g = self._one_graphs[key] = h
         _lib.call("esr_bcg_graph_launch", g, self._stream())
         self.kernel_launches += 1
-        return [self._info(s) for s in self.instances()]
+        return [self._info(s) for s in self._checked(self.instances())]
 
     def _free_graphs(self):
         graphs = getattr(self, "_one_graphs", {})
@@ -523,13 +523,18 @@ class BatchedPCG:
         step() calls - 1), the final recurrence residual, the FP64 true
         residual and the number of residual replacements."""
         self.run(rtol, atol, maxiter, max_rounds)
-        insts = self.instances()
-        if self.solo and insts[0].done == 3:
+        return [self._info(s) for s in self._checked(self.instances())]
+
+    def _checked(self, insts):
+        """``insts``, unless one stopped because a wait on the device ran out
+        (the kernels then stop the instance as in a breakdown)."""
+        if any(s.done == 3 for s in insts):
             from .. import ops
             if ops.device_status(clear=True) & _lib.DEV_WAIT_TIMEOUT:
-                self._solo_comm.zero_()
-                raise RuntimeError("the CTAs of a CG launch timed out waiting for one another")
-        return [self._info(s) for s in insts]
+                if self.solo:
+                    self._solo_comm.zero_()
+                raise RuntimeError("a wait of the CG kernels timed out on the device")
+        return insts
 
     @staticmethod
     def _info(s) -> dict:

@@ -747,7 +747,9 @@ int esr_bcg_init(const esr_batch *B, const double *b64, const void *b, void *x,
  * plus poly_degree polynomial sweeps and 5 GNN launches where those
  * preconditioners are on.  Instances that stop
  * inside the call skip their chunks; the host enqueues calls (e.g. as CUDA
- * graphs) and polls esr_bcg_status between them.  q is scratch [n]. */
+ * graphs) and polls esr_bcg_status between them.  q is scratch [n].  The
+ * sweeps' waits are bounded: on time-out ESR_DEV_WAIT_TIMEOUT is raised and
+ * the instances concerned stop (done = 3). */
 int esr_bcg_iterate(const esr_batch *B, void *x, void *r, void *z, void *p,
                     void *q, int32_t k, void *workspace, void *stream);
 
@@ -758,8 +760,9 @@ int esr_bcg_iterate(const esr_batch *B, void *x, void *r, void *z, void *p,
  * this a solve must not switch (the first direction of a state that
  * esr_bcg_init or esr_bcg_verify left is p = z; q = A z).
  * esr_pcg_solo_ctas: the launch's CTAs on the current device, 0 if the batch
- * does not qualify.  max_width: no slice has more slots (widest row).  comm: esr_pcg_solo_comm_bytes() of device memory, zeroed
- * before its first use and used by one solve at a time.  CTAs wait for one
+ * does not qualify.  max_width: no slice has more slots (widest row).  comm:
+ * esr_pcg_solo_comm_bytes() of device memory, zeroed before its first use and
+ * used by one solve at a time.  CTAs wait for one
  * another with a bounded poll; on time-out ESR_DEV_WAIT_TIMEOUT is raised,
  * the instance stops (done = 3) and comm must be zeroed again. */
 int esr_pcg_solo_ctas(const esr_batch *B);
