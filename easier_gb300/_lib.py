@@ -74,7 +74,7 @@ class Batch(Structure):
                 ("col", c_void_p), ("val", c_void_p), ("diag", c_void_p), ("invdiag", c_void_p),
                 ("val64", c_void_p), ("diag64", c_void_p), ("block_inst", c_void_p), ("inst_block0", c_void_p),
                 ("chunk_tile0", c_void_p), ("chunk_inst", c_void_p), ("inst_chunk0", c_void_p),
-                ("gnn", POINTER(Gnn)), ("poly_tmp", c_void_p), ("poly_degree", c_int32), ("pad_poly_", c_int32)]
+                ("gnn", POINTER(Gnn)), ("poly_tmp", c_void_p), ("poly_degree", c_int32), ("tile_slots", c_int32)]
 
 
 class BcgInst(Structure):

@@ -154,17 +154,19 @@ bcg_init_kernel(BArgs a, const typename P::V *__restrict__ val, const typename P
 // A first direction (refresh != 0: after init or a residual replacement,
 // and the GNN's fallback to Jacobi) is p = z, q = A z.  The GNN's clipped
 // correction is folded into z by bcg_zfix_kernel before.
-// (Three CTAs a SM with two stages each: 24 warps compute; two with three or
-// four stages were slower.  A tile whose slices are wider than eight on average
-// reads its columns and values from memory.)
+// (Three CTAs a SM: 24 warps compute; two with deeper rings were slower.  Where
+// no tile's slices are wider than five on average there is room for a third
+// stage, 90.9 -> 87.3 ms in the case of bcg_stream.cuh, else for two stages of
+// eight; a tile that is wider reads its columns and values from memory.  The
+// update sweep's rings: three stages 89.5 ms, four 91.1, six at three CTAs 92.3.)
 constexpr int kPqCtas = 3, kUpdateCtas = 4;
-constexpr int kPqSlots = 8 * kBThreads;  // slots of a tile's slices that a stage has room for
+constexpr int kPqNarrow = 5 * kBThreads, kPqWide = 8 * kBThreads;  // slots of a tile's slices in a stage
 
-template <class P_>
+template <class P_, int kPqSlots>
 struct PqSweep {
   using P = P_;
   using V = typename P::V;
-  static constexpr int S = 2, K = 1;
+  static constexpr int S = kPqSlots == kPqNarrow ? 3 : 2, K = 1;
   static constexpr uint32_t kSweep = 1;
   static constexpr int kStageBytes = 4 * kTileBytes + 12 * kPqSlots;
   struct Meta {
@@ -268,12 +270,12 @@ struct PqSweep {
   }
 };
 
-template <class P>
+template <class P, int SLOTS>
 __global__ void __launch_bounds__(kStreamThreads, kPqCtas)
 bcg_pq_kernel(BArgs a, const typename P::V *__restrict__ val, const typename P::V *__restrict__ diag,
               const typename P::V *__restrict__ z, typename P::V *__restrict__ p, typename P::V *__restrict__ q,
               bool wide, BcgLayout L) {
-  using OP = PqSweep<P>;
+  using OP = PqSweep<P, SLOTS>;
   extern __shared__ __align__(128) char s_ring[];
   __shared__ StreamShared<P, OP::S, OP::K> s_stream;
   OP op{a, val, diag, z, p, q, wide, {}, L};
@@ -370,7 +372,7 @@ template <class P_>
 struct UpdateSweep {
   using P = P_;
   using V = typename P::V;
-  static constexpr int S = 4, K = 2;
+  static constexpr int S = 3, K = 2;
   static constexpr uint32_t kSweep = 2;
   static constexpr int kStageBytes = 5 * kTileBytes;
   struct Meta {};
@@ -673,12 +675,17 @@ int run_iterate(const esr_batch *B, void *x, void *r, void *z, void *p, void *q,
   for (const void *v : {(const void *)B->col, B->val, B->diag, B->invdiag, (const void *)x, (const void *)r,
                         (const void *)z, (const void *)p, (const void *)q})
     wide = wide && (uintptr_t)v % 16 == 0;
-  constexpr int pq_smem = PqSweep<P>::S * PqSweep<P>::kStageBytes;
+  using Narrow = PqSweep<P, kPqNarrow>;
+  using Wide = PqSweep<P, kPqWide>;
+  const bool narrow = B->tile_slots > 0 && B->tile_slots <= kPqNarrow;
+  const int pq_smem = narrow ? Narrow::S * Narrow::kStageBytes : Wide::S * Wide::kStageBytes;
+  decltype(&bcg_pq_kernel<P, kPqWide>) pq_kernel = nullptr;
+  if constexpr (P::kFusedDirection) pq_kernel = narrow ? bcg_pq_kernel<P, kPqNarrow> : bcg_pq_kernel<P, kPqWide>;
   constexpr int update_smem = UpdateSweep<P>::S * UpdateSweep<P>::kStageBytes;
   cudaError_t e = cudaFuncSetAttribute(bcg_update_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, update_smem);
   if constexpr (P::kFusedDirection)
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(bcg_pq_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, pq_smem);
+      e = cudaFuncSetAttribute(pq_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, pq_smem);
   if (e != cudaSuccess) return esr::cuda_check(e, "esr_bcg_iterate/smem attribute");
   int dev = 0, sms = 0;
   e = cudaGetDevice(&dev);
@@ -706,8 +713,8 @@ int run_iterate(const esr_batch *B, void *x, void *r, void *z, void *p, void *q,
         bcg_pupdate_kernel<P><<<B->grid, kBThreads, 0, s>>>(a, (const V *)z, (V *)p, L);
     }
     if constexpr (P::kFusedDirection)
-      bcg_pq_kernel<P><<<pq_grid, kStreamThreads, pq_smem, s>>>(a, (const V *)B->val, (const V *)B->diag,
-                                                                (const V *)z, (V *)p, (V *)q, wide, L);
+      pq_kernel<<<pq_grid, kStreamThreads, pq_smem, s>>>(a, (const V *)B->val, (const V *)B->diag, (const V *)z,
+                                                         (V *)p, (V *)q, wide, L);
     else
       bcg_spmv_kernel<P><<<B->grid, kBThreads, 0, s>>>(a, (const V *)B->val, (const V *)B->diag, (const V *)p,
                                                        (V *)q, L);

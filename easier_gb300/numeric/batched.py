@@ -227,6 +227,7 @@ class BatchedPCG:
         n = pk.n
         t = lambda a: torch.from_numpy(a).to(dev)
         self.slice_ptr = t(pk.slice_ptr)
+        self._tile_slots = int(np.diff(pk.slice_ptr[::ROWS_PER_BLOCK // 32]).max(initial=0))
         self.col = t(pk.col)
         self.block_inst = t(pk.block_inst)
         self.inst_block0 = t(pk.inst_block0)
@@ -297,7 +298,7 @@ class BatchedPCG:
                                _lib.ptr(self.inst_block0), _lib.ptr(self.chunk_tile0), _lib.ptr(self.chunk_inst),
                                _lib.ptr(self.inst_chunk0),
                                ctypes.pointer(self.gnn_desc) if self.gnn_desc is not None else None,
-                               _lib.ptr(self.poly_tmp), self.poly_degree, 0)
+                               _lib.ptr(self.poly_tmp), self.poly_degree, self._tile_slots)
         self._graphs = {}
         self._free_graphs()
 

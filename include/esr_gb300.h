@@ -704,7 +704,8 @@ typedef struct {
    * omega > 0, an odd d needs omega * lambda_max(D^-1 A) < 2. */
   void *poly_tmp;            /* [2][n] scratch (FP64 or df64), d > 0       */
   int32_t poly_degree;       /* d: SpMV sweeps per application             */
-  int32_t pad_poly_;
+  int32_t tile_slots;        /* no 256-row tile's slices hold more slots (0:
+                                unknown): chooses the streamed sweep's shape */
 } esr_batch;
 
 /* Per-instance device scalars. */
