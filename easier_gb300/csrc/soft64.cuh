@@ -196,8 +196,11 @@ ESR_HD void round_up(uint32_t &mh, uint32_t &ml, uint32_t t, uint32_t r, uint32_
 ESR_HD double product(double a, double b) {
   const uint64_t ua = bits(a), ub = bits(b);
   const uint32_t ha = (uint32_t)(ua >> 32), la = (uint32_t)ua, hb = (uint32_t)(ub >> 32), lb = (uint32_t)ub;
-  // both exponents' top two bits differ: factors within 2^-511 .. 2^512
-  if (((ha ^ (ha << 1)) & (hb ^ (hb << 1)) & 0x40000000u) != 0) {
+  // both exponent fields in 512 .. 1534 (factors in [2^-511, 2^512)): the
+  // result's, with the carry of the mantissas' product or of the rounding (never
+  // both), in 1 .. 2046, always a normal number.  One more on top and 2^512 *
+  // 2^512 would run into the infinity pattern and the sign bit.
+  if ((ha << 1) - (512u << 21) < (1023u << 21) && (hb << 1) - (512u << 21) < (1023u << 21)) {
     const uint32_t ah = shift_left(la, ha, 11) | 0x80000000u, al = la << 11;
     const uint32_t bh = (hb & 0xfffffu) | 0x100000u;
     const uint64_t p00 = (uint64_t)al * lb;
