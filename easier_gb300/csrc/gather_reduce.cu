@@ -9,6 +9,7 @@
 #include <mutex>
 
 #include "esr_internal.h"
+#include "gather_tile.cuh"
 #include "reduce_util.cuh"
 #include "soft64.cuh"
 
@@ -16,25 +17,14 @@ namespace {
 
 constexpr int kThreads = 256;
 
-// Local element -> (row, column) of a tile without a division: j / d for
-// j < 2^16 and 1 <= d < 2^16 is umulhi(j, ceil(2^32 / d)) exactly (the
-// rounding error of the quotient, j * (d - 1) / (d * 2^32), stays below 1/d).
-struct FastDiv {
-  uint32_t d, magic;
-};
-
-inline FastDiv fast_div(uint32_t d) { return FastDiv{d, d > 1 ? (uint32_t)((((uint64_t)1 << 32) + d - 1) / d) : 0u}; }
-
-template <int D>
-__device__ __forceinline__ uint32_t div_by(uint32_t j, FastDiv f) {
-  if (D > 0) return j / (uint32_t)(D > 0 ? D : 1);
-  return f.d > 1 ? __umulhi(j, f.magic) : j;
-}
+using gather::div_by;
+using gather::fast_div;
+using gather::FastDiv;
 
 // ---------------------------------------------------------------- gather --
 // Bound: HBM, given enough loads in flight (index -> row is a chain of two
 // dependent loads) and few enough instructions a vector.  A CTA takes a tile
-// of whole rows (or of up to kGatherCols vectors of long rows, blockIdx.y) of
+// of whole rows (or of up to gather::kCols vectors of long rows, blockIdx.y) of
 // about U * kThreads vectors; a thread requests U indices, then U row
 // vectors, strided so that every store and index load is coalesced.  In a
 // tile of whole rows vector j goes to offset j, and its (row, column) is a
@@ -42,44 +32,13 @@ __device__ __forceinline__ uint32_t div_by(uint32_t j, FastDiv f) {
 // flight a thread, as before, took 59 us for 5.87 M rows of 12 bytes (this
 // form 37, whole rows a thread as below 25: 4.7 TB/s of the bytes it must
 // move).
-constexpr int kGatherCols = 1024;  // vectors of one row a tile takes at most
-
-// O: type of a vector's offset in x (32 bits where x is small enough)
 template <typename V, int D, int U, typename O>
 __global__ void __launch_bounds__(kThreads)
 gather_kernel(const V *__restrict__ x, uint32_t n_in, O vpr, const int32_t *__restrict__ idx, int64_t m,
               V *__restrict__ y, int rows_per_tile, FastDiv cols, int64_t col0) {
-  const int64_t row0 = (int64_t)blockIdx.x * rows_per_tile;
-  const O c0 = D > 0 ? O(0) : (O)(col0 + (int64_t)blockIdx.y * kGatherCols);
-  const uint32_t rows = (uint32_t)(m - row0 < rows_per_tile ? m - row0 : rows_per_tile);
-  const uint32_t width = D > 0 ? (uint32_t)D : (uint32_t)((int64_t)vpr - (int64_t)c0 < cols.d ? (int64_t)vpr - (int64_t)c0 : cols.d);
-  const O row_len = D > 0 ? (O)D : vpr;
-  const uint32_t count = rows * width;  // (a row cut into column blocks: one row a tile, no division)
-  const bool cut = D == 0 && (int64_t)vpr > kGatherCols;
-  const int32_t *__restrict__ ti = idx + row0;
-  V *__restrict__ ty = y + row0 * (int64_t)row_len + (int64_t)c0;
-  for (uint32_t j0 = threadIdx.x; j0 < count; j0 += U * kThreads) {
-    uint32_t s[U], c[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const uint32_t j = j0 + u * kThreads;
-      const uint32_t r = cut ? 0u : div_by<D>(j, cols);
-      c[u] = j - r * width;
-      s[u] = j < count ? (uint32_t)__ldg(ti + r) : 0u;
-    }
-    V v[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u)
-      if (s[u] < n_in) v[u] = x[(O)s[u] * row_len + c0 + c[u]];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const uint32_t j = j0 + u * kThreads;
-      if (j < count) {
-        if (s[u] < n_in) ty[j] = v[u];
-        else esr::raise_status(ESR_DEV_IDX_RANGE);
-      }
-    }
-  }
+  if (!gather::copy_part<V, D, U, O, kThreads>(x, n_in, vpr, idx, m, y, rows_per_tile, cols, col0, blockIdx.x,
+                                               blockIdx.y, threadIdx.x))
+    esr::raise_status(ESR_DEV_IDX_RANGE);
 }
 
 // Rows of D (3) vectors: a thread takes U whole rows, whose vectors go through
@@ -137,13 +96,12 @@ void launch_gather_rows(const V *x, int64_t n_in, const int32_t *idx, int64_t m,
 
 template <typename V, int D, int U>
 void launch_gather_u(const V *x, int64_t n_in, int64_t vpr, const int32_t *idx, int64_t m, V *y, cudaStream_t st) {
-  const int width = (int)(vpr < kGatherCols ? vpr : kGatherCols);
-  const int rows = width >= U * kThreads ? 1 : U * kThreads / width;
+  const int width = gather::tile_width(vpr), rows = gather::tile_rows(width, U * kThreads);
   const int64_t gx = (m + rows - 1) / rows;
   // indices are int32: none of them reaches 2^31
   const uint32_t nin = n_in > ((int64_t)1 << 31) ? (uint32_t)1 << 31 : (uint32_t)n_in;
-  for (int64_t c0 = 0; c0 < vpr; c0 += (int64_t)65535 * kGatherCols) {
-    int64_t gy = (vpr - c0 + kGatherCols - 1) / kGatherCols;
+  for (int64_t c0 = 0; c0 < vpr; c0 += (int64_t)65535 * gather::kCols) {
+    int64_t gy = (vpr - c0 + gather::kCols - 1) / gather::kCols;
     if (gy > 65535) gy = 65535;
     const dim3 g((unsigned)gx, (unsigned)gy);
     if (n_in * vpr < ((int64_t)1 << 31))
