@@ -646,7 +646,9 @@ int run_coop(const esr_sell *A, const T *invdiag, const T *b, T *x, T *r, T *V, 
   int32_t on_chip = smem + (int64_t)cap * restart * (int)sizeof(T) <= kGmSmem ? 1 : 0;
   if (on_chip) smem += cap * restart * (int)sizeof(T);
   const void *fn = (const void *)gm_cycle_kernel<T>;
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  // (the limit belongs to the function, not to this launch: always the largest,
+  // or another thread's smaller system could lower it before this launch)
+  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kGmSmem);
   if (e != cudaSuccess) return esr::cuda_check(e, "esr_gmres_cycle/smem attribute");
   esr_sell a = *A;
   void *args[] = {&a, &invdiag, &b, &x, &r, &V, &w2, &restart, &cap, &on_chip, &cycles, &w};

@@ -263,7 +263,9 @@ extern "C" int esr_pcg_solo_iterate(const esr_batch *B, int32_t max_width, void 
   const bool small = cap <= kSoloThreads && max_width <= 8;
   const void *fn = B->invdiag ? (small ? (const void *)pcg_solo_kernel<true, true> : (const void *)pcg_solo_kernel<true, false>)
                               : (small ? (const void *)pcg_solo_kernel<false, true> : (const void *)pcg_solo_kernel<false, false>);
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  // (the limit belongs to the function, not to this launch: always the largest,
+  // or another thread's smaller system could lower it before this launch)
+  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kSoloSmem);
   if (e != cudaSuccess) return esr::cuda_check(e, "esr_pcg_solo_iterate/smem attribute");
   const double *val = (const double *)B->val, *diag = (const double *)B->diag, *inv = (const double *)B->invdiag;
   GridComm *cm = (GridComm *)comm;
