@@ -304,6 +304,14 @@ inline BArgs bargs(const esr_batch *B) {
 
 __device__ __forceinline__ void retire(BcgLayout L) { atomicSub(&L.head->active, 1); }
 
+// done of an instance one of whose waits gave up: its result is void.  (Kept
+// with the instance, not only in the device status word, which is the whole
+// device's: a breakdown of another solve must not be taken for it.)
+constexpr int kTimedOut = 4;
+__device__ __forceinline__ void give_up(BcgLayout L, int inst) {
+  if (atomicExch(&L.inst[inst].done, kTimedOut) == 0) retire(L);
+}
+
 // tile-grid finish (init / verify kernels: one CTA per tile)
 template <int K>
 __device__ __forceinline__ bool tile_finish(const BArgs &a, int inst, const double (&v)[K], BcgLayout L,

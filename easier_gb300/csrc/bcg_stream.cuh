@@ -28,7 +28,7 @@
 //
 // Every wait is bounded.  A warp that gives up raises ESR_DEV_WAIT_TIMEOUT
 // and leaves; so, in turn, do the others, and the finishing warp stops the
-// instances of the chunks it did not get (done = 3).
+// instances of the chunks it did not get (done = kTimedOut).
 #pragma once
 
 #include "bcg_common.cuh"
@@ -331,7 +331,7 @@ __device__ __forceinline__ void stream_chunks(const BArgs &a, const BcgLayout &L
           op.finish(L.inst[inst], tot);
         }
       }
-      if (!there && lane == 0 && atomicExch(&L.inst[inst].done, 3) == 0) retire(L);
+      if (!there && lane == 0) give_up(L, inst);
     }
   }
 }

@@ -38,9 +38,9 @@ constexpr int kGmMaxRestart = 64;
 struct GmState {
   double rnorm, bnorm, tol, pad0;
   int32_t jend;    // Arnoldi columns of the current cycle
-  int32_t broken;  // breakdown in the current cycle (2: a wait between CTAs timed out)
+  int32_t broken;  // breakdown in the current cycle
   int32_t cycles;
-  int32_t pad1;
+  int32_t timed_out;  // a wait between CTAs gave up (any of them) since the init
   // (the host reads the fields above)
   double H[(kGmMaxRestart + 1) * kGmMaxRestart];  // [i][j] at i * kGmMaxRestart + j
   double y[kGmMaxRestart];
@@ -611,12 +611,15 @@ gm_cycle_kernel(esr_sell A, const T *__restrict__ invdiag, const T *__restrict__
   }
   if (t == 0) {
     sh.cycle = -1;
-    if (!ok) esr::raise_status(ESR_DEV_WAIT_TIMEOUT);
+    if (!ok) {
+      esr::raise_status(ESR_DEV_WAIT_TIMEOUT);
+      atomicExch(&st.timed_out, 1);
+    }
   }
   if (blockIdx.x == 0 && t == 0) {
     st.rnorm = ok ? sh.rnorm : nan("");
     st.jend = columns;
-    st.broken = ok ? sh.broken : 2;
+    st.broken = sh.broken;
     st.cycles += done;
     comm->one.epoch = epoch;
   }
@@ -762,7 +765,7 @@ extern "C" int esr_gmres_read(const void *workspace, esr_gmres_scalars *out, voi
   const GmWork *w = (const GmWork *)workspace;
   struct {
     double rnorm, bnorm, tol, pad0;
-    int32_t jend, broken, cycles, pad1;
+    int32_t jend, broken, cycles, timed_out;
   } h;  // the head of GmState
   cudaError_t e = cudaMemcpyAsync(&h, &w->s, sizeof(h), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -771,7 +774,7 @@ extern "C" int esr_gmres_read(const void *workspace, esr_gmres_scalars *out, voi
   out->bnorm = h.bnorm;
   out->tol = h.tol;
   out->jend = h.jend;
-  out->broken = h.broken;
+  out->broken = h.timed_out ? 2 : h.broken;
   out->cycles = h.cycles;
   out->pad_ = 0;
   return ESR_OK;

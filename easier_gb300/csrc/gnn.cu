@@ -333,7 +333,10 @@ gnn_layer_kernel(BArgs a, GArgs g, const typename P::V *__restrict__ r, const ty
       tc_fence_before();
       __syncthreads();  // sU, sY and the accumulator are reused by the next tile
     }
-    if (stop) break;
+    if (stop) {
+      if (tid == 0) give_up(L, inst);
+      break;
+    }
     if (LAYER == 4) {
       const double v[3] = {bsum<kGThreads>(nr), bsum<kGThreads>(nq), bsum<kGThreads>(jq)};
       double tot[3];

@@ -195,7 +195,10 @@ pcg_solo_kernel(BArgs a, const double *__restrict__ val, const double *__restric
     p[row0 + j] = sp[j];
     q[row0 + j] = sq[j];
   }
-  if (t == 0 && failed) esr::raise_status(ESR_DEV_WAIT_TIMEOUT);
+  if (t == 0 && failed) {  // (any CTA: the others may have got their sums and left)
+    esr::raise_status(ESR_DEV_WAIT_TIMEOUT);
+    give_up(L, 0);
+  }
   if (blockIdx.x == 0 && t == 0) {
     inst.rz = rz;
     inst.rz_jac = rz;
@@ -206,11 +209,7 @@ pcg_solo_kernel(BArgs a, const double *__restrict__ val, const double *__restric
     set_alpha(inst, alpha);
     set_beta(inst, sh.beta);
     comm->epoch = epoch;
-    if (failed) done = 3;
-    if (done) {
-      inst.done = done;
-      retire(L);
-    }
+    if (done && atomicCAS(&inst.done, 0, done) == 0) retire(L);
   }
 }
 

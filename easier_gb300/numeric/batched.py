@@ -31,7 +31,7 @@ import torch
 from .. import _lib, mesh
 
 ROWS_PER_BLOCK = 256
-STATUS = {0: "running", 1: "converged", 2: "maxiter", 3: "breakdown"}
+STATUS = {0: "running", 1: "converged", 2: "maxiter", 3: "breakdown", 4: "timed out"}
 # damping of the polynomial-Jacobi sweeps: fewest iterations on the P1
 # Poisson family at degrees 2 and 4 (the classical 2/3 takes ~5% more
 # iterations there, 1.0 ~20% more)
@@ -472,10 +472,7 @@ class BatchedPCG:
             rounds += 1
             if self.active() == 0 or rounds >= max_rounds:
                 if self.gnn_desc is not None:
-                    from .. import ops
-                    bits = ops.device_status(clear=True)
-                    if bits & _lib.DEV_WAIT_TIMEOUT:
-                        raise RuntimeError("a GNN tensor-core wait timed out on the device")
+                    self._checked(self.instances())
                 return rounds
 
     # ------------------------------------------------- one-launch solve --
@@ -527,14 +524,13 @@ class BatchedPCG:
         return [self._info(s) for s in self._checked(self.instances())]
 
     def _checked(self, insts):
-        """``insts``, unless one stopped because a wait on the device ran out
-        (the kernels then stop the instance as in a breakdown)."""
-        if any(s.done == 3 for s in insts):
-            from .. import ops
-            if ops.device_status(clear=True) & _lib.DEV_WAIT_TIMEOUT:
-                if self.solo:
-                    self._solo_comm.zero_()
-                raise RuntimeError("a wait of the CG kernels timed out on the device")
+        """``insts``, unless one stopped because a wait on the device ran out.
+        (The instance says so itself; the device's status bits stay as they are
+        for whoever asks for them.)"""
+        if any(s.done == 4 for s in insts):
+            if self.solo:
+                self._solo_comm.zero_()
+            raise RuntimeError("a wait of the CG kernels timed out on the device")
         return insts
 
     @staticmethod

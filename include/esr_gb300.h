@@ -717,7 +717,8 @@ typedef struct {
   double rz_jac;     /* r.(invdiag r) of the current residual               */
   double theta;      /* weight of the network's correction in z (GNN mode)  */
   int32_t iters;     /* completed step() calls                              */
-  int32_t done;      /* 0 running, 1 converged, 2 maxiter, 3 breakdown/NaN  */
+  int32_t done;      /* 0 running, 1 converged, 2 maxiter, 3 breakdown/NaN, *
+                      * 4 a wait on the device gave up (result void)        */
   int32_t verified;  /* 1 = FP64 true residual <= tol                       */
   int32_t restarts;  /* residual replacements after a failed verification   */
   int32_t maxiter;
@@ -750,7 +751,7 @@ int esr_bcg_init(const esr_batch *B, const double *b64, const void *b, void *x,
  * inside the call skip their chunks; the host enqueues calls (e.g. as CUDA
  * graphs) and polls esr_bcg_status between them.  q is scratch [n].  The
  * sweeps' waits are bounded: on time-out ESR_DEV_WAIT_TIMEOUT is raised and
- * the instances concerned stop (done = 3). */
+ * the instances concerned stop (done = 4). */
 int esr_bcg_iterate(const esr_batch *B, void *x, void *r, void *z, void *p,
                     void *q, int32_t k, void *workspace, void *stream);
 
@@ -765,7 +766,7 @@ int esr_bcg_iterate(const esr_batch *B, void *x, void *r, void *z, void *p,
  * esr_pcg_solo_comm_bytes() of device memory, zeroed before its first use and
  * used by one solve at a time.  CTAs wait for one
  * another with a bounded poll; on time-out ESR_DEV_WAIT_TIMEOUT is raised,
- * the instance stops (done = 3) and comm must be zeroed again. */
+ * the instance stops (done = 4) and comm must be zeroed again. */
 int esr_pcg_solo_ctas(const esr_batch *B);
 int64_t esr_pcg_solo_comm_bytes(void);
 int esr_pcg_solo_iterate(const esr_batch *B, int32_t max_width, void *x,
