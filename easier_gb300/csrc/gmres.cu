@@ -363,15 +363,6 @@ __device__ __forceinline__ bool many_dots(GmShared &sh, const T *V, int64_t stri
   return sh.failed == 0;
 }
 
-// Barrier of the grid: every thread's earlier global stores are visible to all
-// CTAs afterwards.
-__device__ __forceinline__ bool publish(ExchangeShared &sh, GridComm *comm, uint32_t epoch) {
-  sync_part(0, kSoloThreads);
-  tell_and_wait(sh, comm, epoch, (int)threadIdx.x, kSoloThreads);
-  sync_part(0, kSoloThreads);
-  return sh.failed == 0;
-}
-
 // w - sum_c h[c] V_c[i]
 template <typename T>
 __device__ __forceinline__ double minus_basis(double w, const T *V, int64_t n, int i, const double *h, int count) {

@@ -90,6 +90,15 @@ __device__ __forceinline__ void tell_and_wait(ExchangeShared &sh, GridComm *comm
   fence_gpu();
 }
 
+// Barrier of the grid: every thread's earlier global stores are visible to all
+// CTAs afterwards.
+__device__ __forceinline__ bool publish(ExchangeShared &sh, GridComm *comm, uint32_t epoch) {
+  sync_part(0, kSoloThreads);
+  tell_and_wait(sh, comm, epoch, (int)threadIdx.x, kSoloThreads);
+  sync_part(0, kSoloThreads);
+  return sh.failed == 0;
+}
+
 // Sums v[0..K) over the grid.  Warps 4 k .. 4 k + 3 add the CTA's values of
 // sum k (one warp a scheduler: FP64 adds issue every 64 cycles each), post
 // them and poll the other CTAs' (a warp 64 of them); 32-CTA sums are left in

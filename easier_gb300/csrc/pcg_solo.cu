@@ -8,20 +8,24 @@
 // sums (45 adds a 256-thread block) and on predicated-off multiply-adds of
 // narrow rows.  Here every multiprocessor keeps x, r, p and q of its rows in
 // shared memory (32 bytes a row, up to 7,000 rows) for the whole launch, the
-// matrix streams from L2, and only z goes through memory.  An iteration has
-// two grid exchanges instead of three launches:
-//   p = z + beta p, q = A z + beta q   (A p_new = A z + beta A p_old, as
-//                                       bcg_pq_kernel); p.q   -> exchange
-//   x += alpha p, r -= alpha q, z = M r; r.r, r.z             -> exchange
-// The second exchange also publishes z.  Their kinds alternate, so no CTA posts
-// a word that another may still read; a CTA whose poll gave up
-// raises ESR_DEV_WAIT_TIMEOUT.
-// Measured: FV Poisson, 40,000 rows, 682 iterations 14.1 -> 5.8 ms; P1 grid,
-// 998,001 rows, 2,720 iterations 153 -> 84 ms (31 us an iteration, 23 of them
-// the two sweeps' FP64 instructions; z = M r takes its product to the integer
-// pipes, soft64.cuh).  Between the two the sweeps' and the exchanges' shares
-// trade places; below them only latency is left: about 1,500 cycles from a
-// post to its poll, 700 for the sums of a CTA, 800 for a scalar division.
+// matrix streams from L2, and only p goes through memory.  An iteration has
+// three grid exchanges instead of three launches:
+//   q = A p; p.q                                      -> exchange
+//   x += alpha p, r -= alpha q, z = M r; r.r, r.z     -> exchange
+//   p = z + beta p, published                         -> barrier
+// Each is of another kind than the one before, so no CTA posts a word that
+// another may still read; a CTA whose poll gave up raises ESR_DEV_WAIT_TIMEOUT
+// and stops the instance.
+// (The form p = z + beta p, q = A z + beta q needs one exchange fewer, z being
+// published with r.r: 5.8 ms in place of 6.6 in the first case below, the same
+// time in the second.  But its q drifts from A p: two to four times the launch
+// sequence's distance from CG in extended precision, where this form has 0.9
+// to 1.15 times.)
+// Measured: FV Poisson, 40,000 rows, 682 iterations 14.4 -> 6.6 ms; P1 grid,
+// 998,001 rows, 2,720 iterations 156 -> 88 ms (32 us an iteration, most of them
+// the sweeps' FP64 instructions; z = M r takes its product to the integer
+// pipes, soft64.cuh).  Below them only latency is left: about 1,500 cycles from
+// a post to its poll, 700 for the sums of a CTA, 800 for a scalar division.
 
 #include "bcg_common.cuh"
 #include "grid_exchange.cuh"
@@ -54,16 +58,16 @@ struct HeldRow {
       v[k] = in ? val[b + 32 * k + lane] : 0.0;
     }
   }
-  __device__ __forceinline__ double sum(const double *z) const {
-    double zc[8];
+  __device__ __forceinline__ double sum(const double *p) const {
+    double pc[8];
 #pragma unroll
     for (int k = 0; k < 8; ++k)
-      if (k < w) zc[k] = c[k] >= 0 ? __ldcg(z + c[k]) : 0.0;
+      if (k < w) pc[k] = c[k] >= 0 ? __ldcg(p + c[k]) : 0.0;
     double acc = 0.0;
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
       if (k >= w) break;  // (uniform in the warp)
-      if (c[k] >= 0) acc = fma(v[k], zc[k], acc);
+      if (c[k] >= 0) acc = fma(v[k], pc[k], acc);
     }
     return acc;
   }
@@ -74,12 +78,12 @@ struct HeldRow {
 template <bool JACOBI, bool SMALL>
 __global__ void __launch_bounds__(kSoloThreads, 1)
 pcg_solo_kernel(BArgs a, const double *__restrict__ val, const double *__restrict__ diag,
-                const double *__restrict__ invdiag, double *__restrict__ x, double *__restrict__ r, double *z,
-                double *__restrict__ p, double *__restrict__ q, int32_t iters, int32_t cap, BcgLayout L,
-                GridComm *comm) {
+                const double *__restrict__ invdiag, double *__restrict__ x, double *__restrict__ r, double *p,
+                int32_t iters, int32_t cap, BcgLayout L, GridComm *comm) {
   extern __shared__ double smem[];
   __shared__ SoloShared sh;
-  double *const sx = smem, *const sr = sx + cap, *const sp = sr + cap, *const sq = sp + cap;
+  // (q = A p until the update, z = M r after it)
+  double *const sx = smem, *const sr = sx + cap, *const sp = sr + cap, *const sqz = sp + cap;
   esr_bcg_inst &inst = L.inst[0];
   if (inst.done) return;
   const int64_t slices = a.n >> 5;
@@ -91,8 +95,7 @@ pcg_solo_kernel(BArgs a, const double *__restrict__ val, const double *__restric
   double rz = inst.rz, rr = inst.rr, pq = inst.pq;
   const double tol = inst.tol, tol2 = tol * tol;
   int count = inst.iters, done = 0;
-  const int maxiter = inst.maxiter;
-  bool first = inst.refresh != 0;
+  const int maxiter = inst.maxiter, count0 = count;
   if (t == 0) {
     sh.beta = inst.beta;
     sh.failed = 0;
@@ -102,10 +105,9 @@ pcg_solo_kernel(BArgs a, const double *__restrict__ val, const double *__restric
     sx[j] = x[row0 + j];
     sr[j] = r[row0 + j];
     sp[j] = p[row0 + j];
-    sq[j] = first ? 0.0 : q[row0 + j];
   }
   __syncthreads();
-  double beta = sh.beta, alpha = 0.0;
+  double alpha = 0.0;
   HeldRow own;
   if constexpr (SMALL) {
     if (warp < nsl) own.load(s0 + warp, lane, a, val, diag, JACOBI ? invdiag : nullptr);
@@ -119,14 +121,11 @@ pcg_solo_kernel(BArgs a, const double *__restrict__ val, const double *__restric
     for (int s = warp; s < nsl; s += kSoloThreads / 32) {
       const int64_t i = (s0 + s) * 32 + lane;
       const int j = s * 32 + lane;
-      const double zi = __ldcg(z + i);
-      double w;
-      if constexpr (SMALL) w = fma(own.diag, zi, own.sum(z));
-      else w = fma(__ldg(diag + i), zi, row_sum(s0 + s, lane, a.n, a.slice_ptr, a.col, val, [&](int32_t c) { return __ldcg(z + c); }));
-      const double pi = first ? zi : fma(beta, sp[j], zi);
-      const double qi = first ? w : fma(beta, sq[j], w);
-      sp[j] = pi;
-      sq[j] = qi;
+      const double pi = sp[j];
+      double qi;
+      if constexpr (SMALL) qi = fma(own.diag, pi, own.sum(p));
+      else qi = fma(__ldg(diag + i), pi, row_sum(s0 + s, lane, a.n, a.slice_ptr, a.col, val, [&](int32_t c) { return __ldcg(p + c); }));
+      sqz[j] = qi;
       v1[0] = fma(pi, qi, v1[0]);
     }
     if (!exchange<1, false>(sh, v1, comm, 0, ++epoch)) break;
@@ -141,29 +140,28 @@ pcg_solo_kernel(BArgs a, const double *__restrict__ val, const double *__restric
       break;
     }
     alpha = sh.alpha;
-    first = false;
     double v2[2] = {0.0, 0.0};
 #pragma unroll 2
     for (int s = warp; s < nsl; s += kSoloThreads / 32) {
       const int64_t i = (s0 + s) * 32 + lane;
       const int j = s * 32 + lane;
       sx[j] = fma(alpha, sp[j], sx[j]);
-      const double ri = fma(-alpha, sq[j], sr[j]);
+      const double ri = fma(-alpha, sqz[j], sr[j]);
       sr[j] = ri;
       double zi = ri;
       if constexpr (JACOBI && SMALL) zi = ri * own.inv;
       else if constexpr (JACOBI) zi = soft64::product(ri, __ldg(invdiag + i));  // (beside the busy FP64 pipe)
-      __stcg(z + i, zi);
+      sqz[j] = zi;
       v2[0] = fma(ri, ri, v2[0]);
       if (JACOBI) v2[1] = fma(ri, zi, v2[1]);
     }
     const soft64::Divisor by_rz(rz);  // (thread 0's)
     bool ok;
     if (JACOBI) {
-      ok = exchange<2, true>(sh, v2, comm, 1, ++epoch);
+      ok = exchange<2, false>(sh, v2, comm, 1, ++epoch);
     } else {  // z = r: one sum
       const double v[1] = {v2[0]};
-      ok = exchange<1, true>(sh, v, comm, 1, ++epoch);
+      ok = exchange<1, false>(sh, v, comm, 1, ++epoch);
     }
     if (!ok) break;
     ++count;
@@ -186,14 +184,20 @@ pcg_solo_kernel(BArgs a, const double *__restrict__ val, const double *__restric
       done = sh.stop;
       break;
     }
-    beta = sh.beta;
+    const double beta = sh.beta;
+#pragma unroll 2
+    for (int s = warp; s < nsl; s += kSoloThreads / 32) {
+      const int j = s * 32 + lane;
+      const double pi = fma(beta, sp[j], sqz[j]);
+      sp[j] = pi;
+      __stcg(p + row0 + j, pi);
+    }
+    if (!publish(sh, comm, ++epoch)) break;
   }
   const bool failed = sh.failed != 0;
   for (int j = t; j < rows; j += kSoloThreads) {
     x[row0 + j] = sx[j];
     r[row0 + j] = sr[j];
-    p[row0 + j] = sp[j];
-    q[row0 + j] = sq[j];
   }
   if (t == 0 && failed) {  // (any CTA: the others may have got their sums and left)
     esr::raise_status(ESR_DEV_WAIT_TIMEOUT);
@@ -205,7 +209,7 @@ pcg_solo_kernel(BArgs a, const double *__restrict__ val, const double *__restric
     inst.rr = rr;
     inst.pq = pq;
     inst.iters = count;
-    inst.refresh = first ? inst.refresh : 0;
+    if (count > count0) inst.refresh = 0;
     set_alpha(inst, alpha);
     set_beta(inst, sh.beta);
     comm->epoch = epoch;
@@ -268,7 +272,7 @@ extern "C" int esr_pcg_solo_iterate(const esr_batch *B, int32_t max_width, void 
   if (e != cudaSuccess) return esr::cuda_check(e, "esr_pcg_solo_iterate/smem attribute");
   const double *val = (const double *)B->val, *diag = (const double *)B->diag, *inv = (const double *)B->invdiag;
   GridComm *cm = (GridComm *)comm;
-  void *args[] = {&a, &val, &diag, &inv, &x, &r, &z, &p, &q, &k, &cap, &L, &cm};
+  void *args[] = {&a, &val, &diag, &inv, &x, &r, &p, &k, &cap, &L, &cm};
   e = cudaLaunchCooperativeKernel(fn, dim3((unsigned)ctas), dim3(kSoloThreads), args, (size_t)smem, esr::as_stream(stream));
   if (e != cudaSuccess) return esr::cuda_check(e, "esr_pcg_solo_iterate");
   return ESR_OK;

@@ -758,9 +758,8 @@ int esr_bcg_iterate(const esr_batch *B, void *x, void *r, void *z, void *p,
 /* Iterations of a batch of one FP64 system (Jacobi or no preconditioner)
  * whose vectors fit the multiprocessors' shared memory (about 1 M rows), as
  * one cooperative launch of up to `k` iterations that keeps them there: the
- * state, scalars and stopping test of esr_bcg_iterate, between which and
- * this a solve must not switch (the first direction of a state that
- * esr_bcg_init or esr_bcg_verify left is p = z; q = A z).
+ * state, iteration (q = A p), scalars and stopping test of esr_bcg_iterate.
+ * q is scratch; z is not written (the next direction is already in p).
  * esr_pcg_solo_ctas: the launch's CTAs on the current device, 0 if the batch
  * does not qualify.  max_width: no slice has more slots (widest row).  comm:
  * esr_pcg_solo_comm_bytes() of device memory, zeroed before its first use and
