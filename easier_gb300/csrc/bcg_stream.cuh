@@ -273,13 +273,14 @@ __device__ __forceinline__ void stream_chunks(const BArgs &a, const BcgLayout &L
         ++tiles;
       }
     }
+    // no copy may land after the CTA has left, whoever gave up (before the stop,
+    // which completes another phase)
+    for (int t = max(tiles - S, 0); t < tiles; ++t) bar_wait(&sh.full[t % S], (t / S) & 1);
     if (ok) ok = bar_wait(&sh.empty[stage], phase ^ 1);
     if (ok && lane == 0) {
       sh.head[stage].bits = kStop;
       bar_arrive(&sh.full[stage]);
     }
-    if (!ok)  // no copy may land after the CTA has left
-      for (int t = max(tiles - S, 0); t < tiles; ++t) bar_wait(&sh.full[t % S], (t / S) & 1);
     return;
   }
   int number = 0;  // finish
