@@ -146,6 +146,8 @@ _SIGS = {
     "esr_pcg_solo_ctas": (c_int, [POINTER(Batch)]),
     "esr_pcg_solo_comm_bytes": (c_int64, []),
     "esr_pcg_solo_iterate": (c_int, [POINTER(Batch), c_int32, _P, _P, _P, _P, _P, c_int32, _P, _P, _P]),
+    "esr_bcg_iterate_timeout": (c_int, [POINTER(Batch), _P, _P, _P, _P, _P, c_int32, _P, _P]),
+    "esr_pcg_solo_iterate_timeout": (c_int, [POINTER(Batch), c_int32, _P, _P, _P, _P, _P, c_int32, _P, _P, _P]),
     "esr_bcg_verify": (c_int, [POINTER(Batch), _P, _P, _P, _P, _P, _P, _P, _P, _P]),
     "esr_bcg_status": (c_int, [_P, c_int32, c_int32, POINTER(c_int32), POINTER(BcgInst), _P]),
     "esr_gnn_apply": (c_int, [POINTER(Batch), _P, _P, _P, _P]),
@@ -158,6 +160,7 @@ _SIGS = {
     "esr_gmres_init": (c_int, [POINTER(Sell), _P, c_double, c_double, _P, _P]),
     "esr_gmres_residual": (c_int, [POINTER(Sell), _P, _P, _P, _P, _P]),
     "esr_gmres_cycles": (c_int, [POINTER(Sell), _P, _P, _P, _P, _P, _P, c_int32, c_int32, _P, _P]),
+    "esr_gmres_cycles_timeout": (c_int, [POINTER(Sell), _P, _P, _P, _P, _P, _P, c_int32, c_int32, _P, _P]),
     "esr_gmres_one_launch": (c_int, [POINTER(Sell), c_int32]),
     "esr_gmres_cycle": (c_int, [POINTER(Sell), _P, _P, _P, _P, _P, _P, c_int32, _P, _P]),
     "esr_gmres_read": (c_int, [_P, POINTER(GmresScalars), _P]),

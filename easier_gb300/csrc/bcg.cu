@@ -270,7 +270,7 @@ struct PqSweep {
   }
 };
 
-template <class P, int SLOTS>
+template <class P, int SLOTS, int POLLS>
 __global__ void __launch_bounds__(kStreamThreads, kPqCtas)
 bcg_pq_kernel(BArgs a, const typename P::V *__restrict__ val, const typename P::V *__restrict__ diag,
               const typename P::V *__restrict__ z, typename P::V *__restrict__ p, typename P::V *__restrict__ q,
@@ -279,7 +279,7 @@ bcg_pq_kernel(BArgs a, const typename P::V *__restrict__ val, const typename P::
   extern __shared__ __align__(128) char s_ring[];
   __shared__ StreamShared<P, OP::S, OP::K> s_stream;
   OP op{a, val, diag, z, p, q, wide, {}, L};
-  stream_chunks(a, L, s_ring, s_stream, op);
+  stream_chunks<POLLS>(a, L, s_ring, s_stream, op);
 }
 
 // ---- the same as two sweeps (FP64 policy): q = A p; p.q; alpha ...
@@ -462,7 +462,7 @@ struct UpdateSweep {
   }
 };
 
-template <class P>
+template <class P, int POLLS>
 __global__ void __launch_bounds__(kStreamThreads, kUpdateCtas)
 bcg_update_kernel(BArgs a, const typename P::V *__restrict__ invdiag, typename P::V *__restrict__ x,
                   typename P::V *__restrict__ r, typename P::V *__restrict__ z, const typename P::V *__restrict__ p,
@@ -471,7 +471,7 @@ bcg_update_kernel(BArgs a, const typename P::V *__restrict__ invdiag, typename P
   extern __shared__ __align__(128) char s_ring[];
   __shared__ StreamShared<P, OP::S, OP::K> s_stream;
   OP op{a, invdiag, x, r, z, p, q, wide, {}, L};
-  stream_chunks(a, L, s_ring, s_stream, op);
+  stream_chunks<POLLS>(a, L, s_ring, s_stream, op);
 }
 
 // ---- polynomial-Jacobi sweep: y_out = y_in + W (r - A y_in), persistent
@@ -664,7 +664,7 @@ int run_init(const esr_batch *B, const double *b64, const void *b, void *x, void
   return ESR_OK;
 }
 
-template <class P>
+template <class P, int POLLS>
 int run_iterate(const esr_batch *B, void *x, void *r, void *z, void *p, void *q, int32_t k, void *ws,
                 cudaStream_t s) {
   using V = typename P::V;
@@ -679,10 +679,10 @@ int run_iterate(const esr_batch *B, void *x, void *r, void *z, void *p, void *q,
   using Wide = PqSweep<P, kPqWide>;
   const bool narrow = B->tile_slots > 0 && B->tile_slots <= kPqNarrow;
   const int pq_smem = narrow ? Narrow::S * Narrow::kStageBytes : Wide::S * Wide::kStageBytes;
-  decltype(&bcg_pq_kernel<P, kPqWide>) pq_kernel = nullptr;
-  if constexpr (P::kFusedDirection) pq_kernel = narrow ? bcg_pq_kernel<P, kPqNarrow> : bcg_pq_kernel<P, kPqWide>;
+  decltype(&bcg_pq_kernel<P, kPqWide, POLLS>) pq_kernel = nullptr;
+  if constexpr (P::kFusedDirection) pq_kernel = narrow ? bcg_pq_kernel<P, kPqNarrow, POLLS> : bcg_pq_kernel<P, kPqWide, POLLS>;
   constexpr int update_smem = UpdateSweep<P>::S * UpdateSweep<P>::kStageBytes;
-  cudaError_t e = cudaFuncSetAttribute(bcg_update_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, update_smem);
+  cudaError_t e = cudaFuncSetAttribute(bcg_update_kernel<P, POLLS>, cudaFuncAttributeMaxDynamicSharedMemorySize, update_smem);
   if constexpr (P::kFusedDirection)
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(pq_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, pq_smem);
@@ -718,7 +718,7 @@ int run_iterate(const esr_batch *B, void *x, void *r, void *z, void *p, void *q,
     else
       bcg_spmv_kernel<P><<<B->grid, kBThreads, 0, s>>>(a, (const V *)B->val, (const V *)B->diag, (const V *)p,
                                                        (V *)q, L);
-    bcg_update_kernel<P><<<update_grid, kStreamThreads, update_smem, s>>>(
+    bcg_update_kernel<P, POLLS><<<update_grid, kStreamThreads, update_smem, s>>>(
         a, (const V *)B->invdiag, (V *)x, (V *)r, (V *)z, (const V *)p, (const V *)q, wide, L);
     if (B->gnn) {
       const int st = esr::gnn_layers(B, r, q, z, ws, s);
@@ -730,6 +730,17 @@ int run_iterate(const esr_batch *B, void *x, void *r, void *z, void *p, void *q,
   }
   ESR_LAUNCH_CHECK("esr_bcg_iterate");
   return ESR_OK;
+}
+
+template <int POLLS>
+int iterate(const esr_batch *B, void *x, void *r, void *z, void *p, void *q, int32_t k, void *workspace, void *stream) {
+  int st = check_batch(B);
+  if (st) return st;
+  if (!x || !r || !z || !p || !q || !workspace) return esr::fail(ESR_ERR_ARG, "null vector");
+  if (k < 0) return esr::fail(ESR_ERR_ARG, "negative iteration count");
+  cudaStream_t s = esr::as_stream(stream);
+  return B->df64 ? run_iterate<PolDF, POLLS>(B, x, r, z, p, q, k, workspace, s)
+                 : run_iterate<PolF64, POLLS>(B, x, r, z, p, q, k, workspace, s);
 }
 
 template <class P>
@@ -820,7 +831,7 @@ int build_graph(const esr_batch *B, const double *b64, const void *b, void *x, v
   // the body
   e = cudaStreamBeginCaptureToGraph(s, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
   if (e != cudaSuccess) return esr::cuda_check(e, "esr_bcg_graph_create/capture body");
-  st = run_iterate<P>(B, x, r, z, p, q, k, ws, s);
+  st = run_iterate<P, kStreamPolls>(B, x, r, z, p, q, k, ws, s);
   if (!st) st = run_verify<P>(B, b64, x, x64, r64, r, z, p, ws, s);
   const int max_bodies = (int)((maxiter + (int64_t)k) / k) * 2 + 16;  // replacements restart instances
   if (!st) {
@@ -911,13 +922,12 @@ extern "C" int esr_bcg_init(const esr_batch *B, const double *b64, const void *b
 
 extern "C" int esr_bcg_iterate(const esr_batch *B, void *x, void *r, void *z, void *p, void *q, int32_t k,
                                void *workspace, void *stream) {
-  int st = check_batch(B);
-  if (st) return st;
-  if (!x || !r || !z || !p || !q || !workspace) return esr::fail(ESR_ERR_ARG, "null vector");
-  if (k < 0) return esr::fail(ESR_ERR_ARG, "negative iteration count");
-  cudaStream_t s = esr::as_stream(stream);
-  return B->df64 ? run_iterate<PolDF>(B, x, r, z, p, q, k, workspace, s)
-                 : run_iterate<PolF64>(B, x, r, z, p, q, k, workspace, s);
+  return iterate<kStreamPolls>(B, x, r, z, p, q, k, workspace, stream);
+}
+
+extern "C" int esr_bcg_iterate_timeout(const esr_batch *B, void *x, void *r, void *z, void *p, void *q, int32_t k,
+                                       void *workspace, void *stream) {
+  return iterate<0>(B, x, r, z, p, q, k, workspace, stream);
 }
 
 extern "C" int esr_bcg_verify(const esr_batch *B, const double *b64, void *x, double *x64, double *r64, void *r,

@@ -37,7 +37,7 @@ namespace {
 
 constexpr int kBWarps = kBThreads / 32;         // warps that compute
 constexpr int kStreamThreads = kBThreads + 64;  // and those that fetch and finish
-constexpr int kStreamPolls = 1 << 22;           // mbarrier polls before giving up
+constexpr int kStreamPolls = 1 << 22;           // polls of a wait before it gives up (POLLS below: 0 in tests of that)
 constexpr int kTileBytes = kBThreads * 8;       // a tile's rows of one vector
 
 __device__ __forceinline__ uint32_t shared_addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -51,8 +51,9 @@ __device__ __forceinline__ void bar_arrive(uint64_t *bar) {
 __device__ __forceinline__ void bar_arrive_expect(uint64_t *bar, int bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(shared_addr(bar)), "r"(bytes) : "memory");
 }
+template <int POLLS>
 __device__ __forceinline__ bool bar_wait(uint64_t *bar, uint32_t parity) {
-  for (int tries = 0; tries < kStreamPolls; ++tries) {
+  for (int tries = 0; tries < POLLS; ++tries) {
     uint32_t done;
     asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
                  : "=r"(done)
@@ -159,8 +160,9 @@ __device__ __forceinline__ void post_sum(ulonglong2 *w, double v, uint32_t tag) 
 }
 
 // Adds to v, in order, the sums at w, w + 32, ... (`count` of them, at most kMailAhead)
+template <int POLLS>
 __device__ __forceinline__ bool read_sums(const ulonglong2 *w, int count, uint32_t tag, double &v) {
-  for (int tries = 0; tries < kStreamPolls; ++tries) {
+  for (int tries = 0; tries < POLLS; ++tries) {
     uint64_t x[kMailAhead], y[kMailAhead];
     bool there = true;
 #pragma unroll
@@ -190,7 +192,7 @@ __device__ __forceinline__ bool read_sums(const ulonglong2 *w, int count, uint32
 //   compute(tile, stage, slice, coefficient, flag)   this thread's row
 //   acc[K]                     the sums so far
 //   finish(inst, tot)          the instance's sums are complete
-template <class OP>
+template <int POLLS, class OP>
 __device__ __forceinline__ void stream_chunks(const BArgs &a, const BcgLayout &L, char *ring,
                                               StreamShared<typename OP::P, OP::S, OP::K> &sh, OP &op) {
   using V = typename OP::V;
@@ -213,7 +215,7 @@ __device__ __forceinline__ void stream_chunks(const BArgs &a, const BcgLayout &L
     int stage = 0, number = 0;
     uint32_t phase = 0;
     while (true) {
-      if (!bar_wait(&sh.full[stage], phase)) return;
+      if (!bar_wait<POLLS>(&sh.full[stage], phase)) return;
       const StageHead h = sh.head[stage];
       if (h.bits & kStop) return;
       V coefficient;
@@ -227,7 +229,7 @@ __device__ __forceinline__ void stream_chunks(const BArgs &a, const BcgLayout &L
       }
       if (h.bits & kLastTile) {
         const int set = number & 1;
-        if (!bar_wait(&sh.parts_empty[set], ((number >> 1) & 1) ^ 1)) return;
+        if (!bar_wait<POLLS>(&sh.parts_empty[set], ((number >> 1) & 1) ^ 1)) return;
 #pragma unroll
         for (int k = 0; k < K; ++k) {
           sh.parts[set][k][threadIdx.x] = thread_part(op.acc[k]);
@@ -262,7 +264,7 @@ __device__ __forceinline__ void stream_chunks(const BArgs &a, const BcgLayout &L
           t1 = __shfl_sync(0xffffffffu, own.t1, k);
         }
         if (left) next = op.meta(t, lane);
-        ok = bar_wait(&sh.empty[stage], phase ^ 1);
+        ok = bar_wait<POLLS>(&sh.empty[stage], phase ^ 1);
         if (!ok) break;
         if (lane == 0) sh.head[stage] = h;
         op.fetch(h.tile, m, ring + stage * OP::kStageBytes, sh.slice[stage], &sh.full[stage], lane);
@@ -275,8 +277,8 @@ __device__ __forceinline__ void stream_chunks(const BArgs &a, const BcgLayout &L
     }
     // no copy may land after the CTA has left, whoever gave up (before the stop,
     // which completes another phase)
-    for (int t = max(tiles - S, 0); t < tiles; ++t) bar_wait(&sh.full[t % S], (t / S) & 1);
-    if (ok) ok = bar_wait(&sh.empty[stage], phase ^ 1);
+    for (int t = max(tiles - S, 0); t < tiles; ++t) bar_wait<kStreamPolls>(&sh.full[t % S], (t / S) & 1);
+    if (ok) ok = bar_wait<POLLS>(&sh.empty[stage], phase ^ 1);
     if (ok && lane == 0) {
       sh.head[stage].bits = kStop;
       bar_arrive(&sh.full[stage]);
@@ -300,7 +302,7 @@ __device__ __forceinline__ void stream_chunks(const BArgs &a, const BcgLayout &L
       // (the instance's count of iterations, and which sweep: no two sweeps
       // of a solve share a tag)
       const uint32_t tag = 2u * (uint32_t)__shfl_sync(0xffffffffu, iters, k) + OP::kSweep;
-      if (ok) ok = bar_wait(&sh.parts_full[set], (number >> 1) & 1);
+      if (ok) ok = bar_wait<POLLS>(&sh.parts_full[set], (number >> 1) & 1);
       bool there = ok;
       if (ok) {
         double sum[K];
@@ -323,7 +325,7 @@ __device__ __forceinline__ void stream_chunks(const BArgs &a, const BcgLayout &L
         for (int j = 0; j < K; ++j) {
           double v = 0.0;
           for (int q = c0 + lane; q < c1; q += 32 * kMailAhead)
-            there = read_sums(L.mail + j * (int64_t)a.nchunks + q, (c1 - q + 31) / 32, tag, v) && there;
+            there = read_sums<POLLS>(L.mail + j * (int64_t)a.nchunks + q, (c1 - q + 31) / 32, tag, v) && there;
           tot[j] = warp_total(v);
         }
         there = __all_sync(0xffffffffu, there);

@@ -291,7 +291,7 @@ struct GmShared : ExchangeShared {
 
 // V^T w over the grid for columns 0 .. columns (and w.w if `square`): into
 // sh.h, past a barrier.  V: the CTA's rows, columns `stride` apart.
-template <typename T>
+template <typename T, int POLLS>
 __device__ __forceinline__ bool many_dots(GmShared &sh, const T *V, int64_t stride, int rows, const double *ws,
                                           int columns, bool square, GmComm *comm, uint32_t epoch) {
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31, grid = (int)gridDim.x, me = (int)blockIdx.x;
@@ -332,7 +332,7 @@ __device__ __forceinline__ bool many_dots(GmShared &sh, const T *V, int64_t stri
   for (int i = me + (kWarps - 1 - warp) * grid; i < count; i += kWarps * grid) {
     double v[kSoloMaxCtas / 32], b = 0.0;
     bool got = false;
-    for (int tries = 0; tries < kSoloPolls && !got; ++tries) {
+    for (int tries = 0; tries < POLLS && !got; ++tries) {
       got = true;
 #pragma unroll
       for (int q = 0; q < kSoloMaxCtas / 32; ++q) {
@@ -356,7 +356,7 @@ __device__ __forceinline__ bool many_dots(GmShared &sh, const T *V, int64_t stri
   }
   if (t < count) {
     double h;
-    if (!poll(&comm->total[me][t], true, false, epoch, h)) sh.failed = 1;
+    if (!poll<POLLS>(&comm->total[me][t], true, false, epoch, h)) sh.failed = 1;
     sh.h[t] = h;
   }
   sync_part(0, kSoloThreads);
@@ -439,7 +439,7 @@ __device__ __forceinline__ void least_squares(GmShared &sh, double *R, int resta
   if (lane == 0) sh.solved = 1;
 }
 
-template <typename T>
+template <typename T, int POLLS>
 __global__ void __launch_bounds__(kGmThreads2, 1)
 gm_cycle_kernel(esr_sell A, const T *__restrict__ invdiag, const T *__restrict__ b, T *x, T *r, T *Vg, T *zs,
                 int32_t restart, int32_t cap, int32_t on_chip, int32_t cycles, GmWork *work) {
@@ -521,11 +521,11 @@ gm_cycle_kernel(esr_sell A, const T *__restrict__ invdiag, const T *__restrict__
         }
       }
       sync_part(0, kSoloThreads);
-      if (!(ok = many_dots<T>(sh, V, stride, rows, ws, j + 1, false, comm, ++epoch))) break;
+      if (!(ok = many_dots<T, POLLS>(sh, V, stride, rows, ws, j + 1, false, comm, ++epoch))) break;
       const double h1 = t <= j ? sh.h[t] : 0.0;
       for (int l = t; l < rows; l += kSoloThreads) ws[l] = minus_basis<T>(ws[l], V, stride, l, sh.h, j + 1);
       sync_part(0, kSoloThreads);
-      if (!(ok = many_dots<T>(sh, V, stride, rows, ws, j + 1, true, comm, ++epoch))) break;
+      if (!(ok = many_dots<T, POLLS>(sh, V, stride, rows, ws, j + 1, true, comm, ++epoch))) break;
       if (t <= j) R[j * (restart + 1) + t] = h1 + sh.h[t];
       if (warp == kSoloThreads / 32 - 1) {  // the norm, beside the other warps' rows
         double hh = lane <= j ? sh.h[lane] * sh.h[lane] : 0.0;
@@ -548,9 +548,9 @@ gm_cycle_kernel(esr_sell A, const T *__restrict__ invdiag, const T *__restrict__
         if (j + 1 < restart)
           __stcg(zs + row0 + l, sizeof(T) == 8 && invdiag ? (T)(w * (double)__ldg(invdiag + row0 + l)) : (T)w);
       }
-      if (!(ok = publish(sh, &comm->one, ++epoch))) break;
+      if (!(ok = publish<POLLS>(sh, &comm->one, ++epoch))) break;
       if (sh.again) {
-        if (!(ok = exchange<1, false>(sh, v, &comm->one, 0, ++epoch))) break;
+        if (!(ok = exchange<1, false, POLLS>(sh, v, &comm->one, 0, ++epoch))) break;
         if (t == 0) {
           const double hn = sqrt(grid_sum(sh, 0));
           R[j * (restart + 1) + j + 1] = hn;
@@ -582,7 +582,7 @@ gm_cycle_kernel(esr_sell A, const T *__restrict__ invdiag, const T *__restrict__
       const T d = (T)-minus_basis<T>(0.0, V, stride, l, sh.y, columns);
       x[i] = (T)((double)x[i] + (invdiag ? (double)(T)((double)d * (double)__ldg(invdiag + i)) : (double)d));
     }
-    if (!(ok = publish(sh, &comm->one, ++epoch))) break;
+    if (!(ok = publish<POLLS>(sh, &comm->one, ++epoch))) break;
     double rr[1] = {0.0};
     for (int s = warp; s < nsl; s += kSoloThreads / 32) {
       const int64_t i = row0 + s * 32 + lane;
@@ -594,7 +594,7 @@ gm_cycle_kernel(esr_sell A, const T *__restrict__ invdiag, const T *__restrict__
         rr[0] = fma((double)ri, (double)ri, rr[0]);
       }
     }
-    if (!(ok = exchange<1, true>(sh, rr, &comm->one, 2, ++epoch))) break;
+    if (!(ok = exchange<1, true, POLLS>(sh, rr, &comm->one, 2, ++epoch))) break;
     if (t == 0) sh.rnorm = sqrt(grid_sum(sh, 0));
     ++done;
     sync_part(0, kSoloThreads);
@@ -633,13 +633,13 @@ int cycle_ctas(int64_t n, int32_t restart, int *cap_out) {
   return (int)g;
 }
 
-template <typename T>
+template <typename T, int POLLS>
 int run_coop(const esr_sell *A, const T *invdiag, const T *b, T *x, T *r, T *V, T *w2, int32_t restart, GmWork *w,
              int ctas, int cap, int32_t cycles, cudaStream_t s) {
   int smem = (cap + restart * (restart + 1)) * (int)sizeof(double);
   int32_t on_chip = smem + (int64_t)cap * restart * (int)sizeof(T) <= kGmSmem ? 1 : 0;
   if (on_chip) smem += cap * restart * (int)sizeof(T);
-  const void *fn = (const void *)gm_cycle_kernel<T>;
+  const void *fn = (const void *)gm_cycle_kernel<T, POLLS>;
   // (the limit belongs to the function, not to this launch: always the largest,
   // or another thread's smaller system could lower it before this launch)
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kGmSmem);
@@ -659,13 +659,13 @@ int check(const esr_sell *A, int32_t restart) {
   return ESR_OK;
 }
 
-template <typename T>
+template <typename T, int POLLS>
 int run_cycle(const esr_sell *A, const T *invdiag, const T *b, T *x, T *r, T *V, T *w2, int32_t restart,
               int32_t cycles, GmWork *w, cudaStream_t s) {
   const int64_t n = A->n;
   int cap = 0;
   if (const int ctas = cycle_ctas(n, restart, &cap))
-    return run_coop<T>(A, invdiag, b, x, r, V, w2, restart, w, ctas, cap, cycles, s);
+    return run_coop<T, POLLS>(A, invdiag, b, x, r, V, w2, restart, w, ctas, cap, cycles, s);
   if (cycles != 1) return esr::fail(ESR_ERR_UNSUPPORTED, "several GMRES cycles a call need the one-launch cycle");
   const int g = grid_for(n);
   gm_initv_kernel<T><<<g, kGmThreads, 0, s>>>(n, r, V, w);
@@ -680,6 +680,22 @@ int run_cycle(const esr_sell *A, const T *invdiag, const T *b, T *x, T *r, T *V,
   gm_resid_kernel<T><<<g, kGmThreads, 0, s>>>(*A, b, x, r, w);
   ESR_LAUNCH_CHECK("esr_gmres_cycle");
   return ESR_OK;
+}
+
+template <int POLLS>
+int run_cycles(const esr_sell *A, const void *invdiag, const void *b, void *x, void *r, void *V, void *w2,
+               int32_t restart, int32_t cycles, void *workspace, void *stream) {
+  int st = check(A, restart);
+  if (st) return st;
+  if (!b || !x || !r || !V || !w2 || !workspace) return esr::fail(ESR_ERR_ARG, "null vector");
+  if (cycles < 1) return esr::fail(ESR_ERR_ARG, "cycles must be positive");
+  cudaStream_t s = esr::as_stream(stream);
+  GmWork *w = (GmWork *)workspace;
+  if (A->dtype == ESR_F64)
+    return run_cycle<double, POLLS>(A, (const double *)invdiag, (const double *)b, (double *)x, (double *)r, (double *)V,
+                                    (double *)w2, restart, cycles, w, s);
+  return run_cycle<float, POLLS>(A, (const float *)invdiag, (const float *)b, (float *)x, (float *)r, (float *)V,
+                                 (float *)w2, restart, cycles, w, s);
 }
 
 }  // namespace
@@ -732,17 +748,13 @@ extern "C" int esr_gmres_residual(const esr_sell *A, const void *b, const void *
 
 extern "C" int esr_gmres_cycles(const esr_sell *A, const void *invdiag, const void *b, void *x, void *r, void *V,
                                 void *w2, int32_t restart, int32_t cycles, void *workspace, void *stream) {
-  int st = check(A, restart);
-  if (st) return st;
-  if (!b || !x || !r || !V || !w2 || !workspace) return esr::fail(ESR_ERR_ARG, "null vector");
-  if (cycles < 1) return esr::fail(ESR_ERR_ARG, "cycles must be positive");
-  cudaStream_t s = esr::as_stream(stream);
-  GmWork *w = (GmWork *)workspace;
-  if (A->dtype == ESR_F64)
-    return run_cycle<double>(A, (const double *)invdiag, (const double *)b, (double *)x, (double *)r, (double *)V,
-                             (double *)w2, restart, cycles, w, s);
-  return run_cycle<float>(A, (const float *)invdiag, (const float *)b, (float *)x, (float *)r, (float *)V,
-                          (float *)w2, restart, cycles, w, s);
+  return run_cycles<kSoloPolls>(A, invdiag, b, x, r, V, w2, restart, cycles, workspace, stream);
+}
+
+extern "C" int esr_gmres_cycles_timeout(const esr_sell *A, const void *invdiag, const void *b, void *x, void *r,
+                                        void *V, void *w2, int32_t restart, int32_t cycles, void *workspace,
+                                        void *stream) {
+  return run_cycles<0>(A, invdiag, b, x, r, V, w2, restart, cycles, workspace, stream);
 }
 
 extern "C" int esr_gmres_cycle(const esr_sell *A, const void *invdiag, const void *b, void *x, void *r, void *V,

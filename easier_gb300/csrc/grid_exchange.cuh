@@ -20,7 +20,7 @@ namespace {
 
 constexpr int kSoloThreads = 512;  // threads that take part
 constexpr int kSoloMaxCtas = 256;
-constexpr int kSoloPolls = 1 << 24;  // (about ten seconds)
+constexpr int kSoloPolls = 1 << 24;  // (about ten seconds; POLLS below: 0 in tests of the giving up)
 
 struct GridComm {
   uint32_t epoch;  // exchanges done by earlier launches
@@ -36,9 +36,10 @@ __device__ __forceinline__ void post(ulonglong2 *w, double v, uint32_t epoch) {
 }
 
 // Polls the words at w (if a) and w + 128 (if b) together; their sum in v.
+template <int POLLS>
 __device__ __forceinline__ bool poll(const ulonglong2 *w, bool a, bool b, uint32_t epoch, double &v) {
   uint64_t x0 = 0, x1 = 0, y0 = 0, y1 = 0;
-  for (int tries = 0; tries < kSoloPolls; ++tries) {
+  for (int tries = 0; tries < POLLS; ++tries) {
     if (a) asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(x0), "=l"(x1) : "l"(w) : "memory");
     if (b) asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(y0), "=l"(y1) : "l"(w + 128) : "memory");
     const bool got_a = !a || ((uint32_t)(x0 >> 32) == epoch && (uint32_t)(x1 >> 32) == epoch);
@@ -74,6 +75,7 @@ struct ExchangeShared {
 
 // Threads first .. of `threads` of a CTA whose stores are done (past a barrier)
 // tell all CTAs so and wait for the same from them.
+template <int POLLS>
 __device__ __forceinline__ void tell_and_wait(ExchangeShared &sh, GridComm *comm, uint32_t epoch, int first,
                                               int threads) {
   const int grid = (int)gridDim.x;
@@ -83,7 +85,7 @@ __device__ __forceinline__ void tell_and_wait(ExchangeShared &sh, GridComm *comm
     asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(&comm->ready[to][blockIdx.x]), "r"(epoch) : "memory");
   for (int i = first; i < grid; i += threads) {
     uint32_t e = epoch - 1;  // (a CTA ahead may already have told of a later exchange)
-    for (int tries = 0; tries < kSoloPolls && (int32_t)(e - epoch) < 0; ++tries)
+    for (int tries = 0; tries < POLLS && (int32_t)(e - epoch) < 0; ++tries)
       asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(e) : "l"(&comm->ready[blockIdx.x][i]) : "memory");
     if ((int32_t)(e - epoch) < 0) sh.failed = 1;
   }
@@ -92,9 +94,10 @@ __device__ __forceinline__ void tell_and_wait(ExchangeShared &sh, GridComm *comm
 
 // Barrier of the grid: every thread's earlier global stores are visible to all
 // CTAs afterwards.
+template <int POLLS>
 __device__ __forceinline__ bool publish(ExchangeShared &sh, GridComm *comm, uint32_t epoch) {
   sync_part(0, kSoloThreads);
-  tell_and_wait(sh, comm, epoch, (int)threadIdx.x, kSoloThreads);
+  tell_and_wait<POLLS>(sh, comm, epoch, (int)threadIdx.x, kSoloThreads);
   sync_part(0, kSoloThreads);
   return sh.failed == 0;
 }
@@ -105,7 +108,7 @@ __device__ __forceinline__ bool publish(ExchangeShared &sh, GridComm *comm, uint
 // sh.cta, past a barrier (grid_sum() adds them).  PUBLISH: every thread's
 // earlier global stores are visible to all CTAs afterwards (warps 8 .. 15).
 // False: a poll gave up.
-template <int K, bool PUBLISH>
+template <int K, bool PUBLISH, int POLLS>
 __device__ __forceinline__ bool exchange(ExchangeShared &sh, const double (&v)[K], GridComm *comm, int first,
                                          uint32_t epoch) {
   const int t = threadIdx.x, g = t >> 7, u = t & 127, lane = t & 31, grid = (int)gridDim.x;
@@ -120,11 +123,11 @@ __device__ __forceinline__ bool exchange(ExchangeShared &sh, const double (&v)[K
     const double b = (sh.warp[g][0] + sh.warp[g][1]) + (sh.warp[g][2] + sh.warp[g][3]);
     for (int to = u; to < grid; to += 128) post(&comm->mail[first + g][to][blockIdx.x], b, epoch);
     double two;
-    if (!poll(&comm->mail[first + g][blockIdx.x][u], u < grid, u + 128 < grid, epoch, two)) sh.failed = 1;
+    if (!poll<POLLS>(&comm->mail[first + g][blockIdx.x][u], u < grid, u + 128 < grid, epoch, two)) sh.failed = 1;
     const double m = warp_sum(two);
     if (lane == 0) sh.cta[g][u >> 5] = m;
   } else if (PUBLISH && t >= 256) {
-    tell_and_wait(sh, comm, epoch, t - 256, 256);
+    tell_and_wait<POLLS>(sh, comm, epoch, t - 256, 256);
   }
   sync_part(0, kSoloThreads);
   return sh.failed == 0;

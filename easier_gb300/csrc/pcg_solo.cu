@@ -75,7 +75,7 @@ struct HeldRow {
 
 // SMALL: at most one slice a warp, of at most eight slots: its matrix stays in
 // registers.
-template <bool JACOBI, bool SMALL>
+template <bool JACOBI, bool SMALL, int POLLS>
 __global__ void __launch_bounds__(kSoloThreads, 1)
 pcg_solo_kernel(BArgs a, const double *__restrict__ val, const double *__restrict__ diag,
                 const double *__restrict__ invdiag, double *__restrict__ x, double *__restrict__ r, double *p,
@@ -128,7 +128,7 @@ pcg_solo_kernel(BArgs a, const double *__restrict__ val, const double *__restric
       sqz[j] = qi;
       v1[0] = fma(pi, qi, v1[0]);
     }
-    if (!exchange<1, false>(sh, v1, comm, 0, ++epoch)) break;
+    if (!exchange<1, false, POLLS>(sh, v1, comm, 0, ++epoch)) break;
     if (t == 0) {
       pq = grid_sum(sh, 0);
       sh.stop = (!(pq != 0.0) || !isfinite(pq)) ? 3 : 0;
@@ -158,10 +158,10 @@ pcg_solo_kernel(BArgs a, const double *__restrict__ val, const double *__restric
     const soft64::Divisor by_rz(rz);  // (thread 0's)
     bool ok;
     if (JACOBI) {
-      ok = exchange<2, false>(sh, v2, comm, 1, ++epoch);
+      ok = exchange<2, false, POLLS>(sh, v2, comm, 1, ++epoch);
     } else {  // z = r: one sum
       const double v[1] = {v2[0]};
-      ok = exchange<1, false>(sh, v, comm, 1, ++epoch);
+      ok = exchange<1, false, POLLS>(sh, v, comm, 1, ++epoch);
     }
     if (!ok) break;
     ++count;
@@ -192,7 +192,7 @@ pcg_solo_kernel(BArgs a, const double *__restrict__ val, const double *__restric
       sp[j] = pi;
       __stcg(p + row0 + j, pi);
     }
-    if (!publish(sh, comm, ++epoch)) break;
+    if (!publish<POLLS>(sh, comm, ++epoch)) break;
   }
   const bool failed = sh.failed != 0;
   for (int j = t; j < rows; j += kSoloThreads) {
@@ -236,6 +236,37 @@ int device_sms(int *sms) {
   return e == cudaSuccess ? ESR_OK : esr::cuda_check(e, "esr_pcg_solo");
 }
 
+template <int POLLS>
+int run_solo(const esr_batch *B, int32_t max_width, void *x, void *r, void *z, void *p, void *q, int32_t k,
+             void *workspace, void *comm, void *stream) {
+  int st = check_batch(B);
+  if (st) return st;
+  if (!x || !r || !z || !p || !q || !workspace || !comm) return esr::fail(ESR_ERR_ARG, "null vector");
+  if (k < 0) return esr::fail(ESR_ERR_ARG, "negative iteration count");
+  const int ctas = esr_pcg_solo_ctas(B);
+  if (!ctas) return esr::fail(ESR_ERR_UNSUPPORTED, "esr_pcg_solo_iterate: one FP64 system that fits the chip's shared memory");
+  if (k == 0) return ESR_OK;
+  BcgLayout L = layout_of(workspace, B->ninst, B->nchunks);
+  BArgs a = bargs(B);
+  const int64_t slices = B->n >> 5;
+  int32_t cap = (int32_t)((slices + ctas - 1) / ctas * 32);
+  const int smem = cap * 4 * (int)sizeof(double);
+  const bool small = cap <= kSoloThreads && max_width <= 8;
+  const void *fn =
+      B->invdiag ? (small ? (const void *)pcg_solo_kernel<true, true, POLLS> : (const void *)pcg_solo_kernel<true, false, POLLS>)
+                 : (small ? (const void *)pcg_solo_kernel<false, true, POLLS> : (const void *)pcg_solo_kernel<false, false, POLLS>);
+  // (the limit belongs to the function, not to this launch: always the largest,
+  // or another thread's smaller system could lower it before this launch)
+  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kSoloSmem);
+  if (e != cudaSuccess) return esr::cuda_check(e, "esr_pcg_solo_iterate/smem attribute");
+  const double *val = (const double *)B->val, *diag = (const double *)B->diag, *inv = (const double *)B->invdiag;
+  GridComm *cm = (GridComm *)comm;
+  void *args[] = {&a, &val, &diag, &inv, &x, &r, &p, &k, &cap, &L, &cm};
+  e = cudaLaunchCooperativeKernel(fn, dim3((unsigned)ctas), dim3(kSoloThreads), args, (size_t)smem, esr::as_stream(stream));
+  if (e != cudaSuccess) return esr::cuda_check(e, "esr_pcg_solo_iterate");
+  return ESR_OK;
+}
+
 }  // namespace
 
 ESR_DEFINE_STATUS_READER(esr_status_pcg_solo)
@@ -251,29 +282,10 @@ extern "C" int64_t esr_pcg_solo_comm_bytes(void) { return (int64_t)sizeof(GridCo
 
 extern "C" int esr_pcg_solo_iterate(const esr_batch *B, int32_t max_width, void *x, void *r, void *z, void *p, void *q,
                                     int32_t k, void *workspace, void *comm, void *stream) {
-  int st = check_batch(B);
-  if (st) return st;
-  if (!x || !r || !z || !p || !q || !workspace || !comm) return esr::fail(ESR_ERR_ARG, "null vector");
-  if (k < 0) return esr::fail(ESR_ERR_ARG, "negative iteration count");
-  const int ctas = esr_pcg_solo_ctas(B);
-  if (!ctas) return esr::fail(ESR_ERR_UNSUPPORTED, "esr_pcg_solo_iterate: one FP64 system that fits the chip's shared memory");
-  if (k == 0) return ESR_OK;
-  BcgLayout L = layout_of(workspace, B->ninst, B->nchunks);
-  BArgs a = bargs(B);
-  const int64_t slices = B->n >> 5;
-  int32_t cap = (int32_t)((slices + ctas - 1) / ctas * 32);
-  const int smem = cap * 4 * (int)sizeof(double);
-  const bool small = cap <= kSoloThreads && max_width <= 8;
-  const void *fn = B->invdiag ? (small ? (const void *)pcg_solo_kernel<true, true> : (const void *)pcg_solo_kernel<true, false>)
-                              : (small ? (const void *)pcg_solo_kernel<false, true> : (const void *)pcg_solo_kernel<false, false>);
-  // (the limit belongs to the function, not to this launch: always the largest,
-  // or another thread's smaller system could lower it before this launch)
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kSoloSmem);
-  if (e != cudaSuccess) return esr::cuda_check(e, "esr_pcg_solo_iterate/smem attribute");
-  const double *val = (const double *)B->val, *diag = (const double *)B->diag, *inv = (const double *)B->invdiag;
-  GridComm *cm = (GridComm *)comm;
-  void *args[] = {&a, &val, &diag, &inv, &x, &r, &p, &k, &cap, &L, &cm};
-  e = cudaLaunchCooperativeKernel(fn, dim3((unsigned)ctas), dim3(kSoloThreads), args, (size_t)smem, esr::as_stream(stream));
-  if (e != cudaSuccess) return esr::cuda_check(e, "esr_pcg_solo_iterate");
-  return ESR_OK;
+  return run_solo<kSoloPolls>(B, max_width, x, r, z, p, q, k, workspace, comm, stream);
+}
+
+extern "C" int esr_pcg_solo_iterate_timeout(const esr_batch *B, int32_t max_width, void *x, void *r, void *z, void *p,
+                                            void *q, int32_t k, void *workspace, void *comm, void *stream) {
+  return run_solo<0>(B, max_width, x, r, z, p, q, k, workspace, comm, stream);
 }

@@ -810,6 +810,22 @@ int esr_gnn_apply(const esr_batch *B, const void *r, void *z, void *workspace,
  * Test hook (no reference counterpart). */
 int esr_wait_selftest(int32_t limit_polls, int32_t *gave_up_dev, void *stream);
 
+/* esr_bcg_iterate, esr_pcg_solo_iterate and esr_gmres_cycles in which every
+ * wait between CTAs and warps gives up at once, and so leaves what a time-out
+ * leaves (done = 4, broken = 2, ESR_DEV_WAIT_TIMEOUT).  The context stays
+ * usable.  Test hooks (no reference counterpart). */
+int esr_bcg_iterate_timeout(const esr_batch *B, void *x, void *r, void *z,
+                            void *p, void *q, int32_t k, void *workspace,
+                            void *stream);
+int esr_pcg_solo_iterate_timeout(const esr_batch *B, int32_t max_width,
+                                 void *x, void *r, void *z, void *p, void *q,
+                                 int32_t k, void *workspace, void *comm,
+                                 void *stream);
+int esr_gmres_cycles_timeout(const esr_sell *A, const void *invdiag,
+                             const void *b, void *x, void *r, void *V,
+                             void *w2, int32_t restart, int32_t cycles,
+                             void *workspace, void *stream);
+
 /* Running-instance count and (if inst_out) the per-instance scalars, to
  * host memory; synchronises `stream`. */
 int esr_bcg_status(const void *workspace, int32_t ninst, int32_t nchunks,
