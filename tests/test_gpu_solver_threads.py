@@ -63,3 +63,23 @@ def test_gmres_cycles_of_two_sizes():
         eng.solve(b, x, r, 0.0, None, 1)
         calls.append(lambda eng=eng, b=b, x=x, r=r: eng._cycle_call(b, x, r, 1))
     _both(calls, 500)
+
+
+def test_solves_on_two_streams_at_once():
+    """Two threads, a stream each: cooperative launches of either wait until
+    all of their CTAs can run."""
+    engines = [BatchedPCG([_chain(n)], precision="fp64") for n in (40_000, 60_000)]
+    assert all(e.solo for e in engines)
+    first = []
+    for e in engines:
+        info = e.solve(rtol=1e-10)
+        first.append((info, e.solution(0).clone()))
+    torch.cuda.synchronize()
+
+    def solve(e, want, x, stream):
+        with torch.cuda.stream(stream):
+            e.reset()
+            assert e.solve(rtol=1e-10) == want and torch.equal(e.solution(0), x)
+
+    streams = [torch.cuda.Stream() for _ in engines]
+    _both([lambda a=(e, *f, s): solve(*a) for e, f, s in zip(engines, first, streams)], 40)
