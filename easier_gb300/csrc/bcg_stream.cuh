@@ -16,12 +16,12 @@
 //
 // Measured on 48 P1 meshes of 32 to 384 cells a side (2.35 M rows, 1,480
 // iterations, double-float): 118.9 -> 85.7 ms, an iteration of all of them
-// 78 us where the copy rate allows 56 (91.0 ms when the forms below were tried).  What bounds it now: in the direction
+// 78 us where the copy rate allows 56.  What bounds it now: in the direction
 // sweep the arithmetic's latency (2,400 of 3,500 cycles a tile, the gathers of
 // z with it) at the 24 computing warps that the rings leave room for, in the
 // update sweep the copies' latency at either end (13,000 of 40,000 cycles).
-// Slower were: gathers loaded a tile ahead, which takes deeper rings and so 16
-// warps a SM (108 ms); copies issued by the computing warps, an array each
+// Slower, against 91.0 ms with the rings of that time, were: gathers loaded a
+// tile ahead, which takes deeper rings and so 16 warps a SM (108 ms); copies issued by the computing warps, an array each
 // (117 ms: a copy takes its warp 200 cycles to issue); no rings but the next
 // tile's columns in registers (199 ms: spills); the next sweep launched early
 // (91.3: no gain inside a captured graph).

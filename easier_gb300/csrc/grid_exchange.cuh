@@ -4,8 +4,8 @@
 // hold 32 bits of the double and the exchange's number; every CTA polls its
 // own mailbox and adds the sums itself in the same order, so all take the same
 // decisions and no second barrier distributes the result.  That its global
-// stores are done a CTA tells with a word of its own, posted by other warps
-// behind a fence while the sums are added.  A word is posted again only after
+// stores are done a CTA tells with a word of its own, posted behind a fence: by
+// other warps while the sums are added, or in a barrier of its own (publish).  A word is posted again only after
 // an exchange that everybody's reading of the last one precedes.  (One set of
 // words that all CTAs poll: 9,000 cycles a poll, 23,000 sector reads a round
 // on twenty lines; mailboxes: 1,500.)  Polls are bounded: a CTA that gives up

@@ -251,8 +251,9 @@ struct SlotsG {  // face slots in global memory, [width][nc]
   const T *sx, *sy, *alpha, *area, *inv_area;
 };
 
-// delta (swe_main.py:87-119) of cell i given the stage state `s`.
-template <typename T, int W, bool EXACT, bool FIRST>
+// Face slot k of cell i given the stage state `s`: a neighbour's flux or a wall.
+// FIRST: the sums are still zero.
+template <typename T, bool EXACT, bool FIRST>
 __device__ __forceinline__ void slot_sums(int k, int64_t i, int64_t nc, const SlotsG<T> &g, const T *s,
                                           const Vec4<T> own, Acc3<T> &acc, bool &walls) {
   const int32_t j = __ldg(g.nbr + k * nc + i);
@@ -270,20 +271,21 @@ __device__ __forceinline__ void slot_sums(int k, int64_t i, int64_t nc, const Sl
   }
 }
 
+// delta (swe_main.py:87-119) of cell i.
 template <typename T, int W, bool EXACT>
 __device__ __forceinline__ Vec4<T> cell_delta(int64_t i, int64_t nc, const SlotsG<T> &g, const T *s,
                                               const Vec4<T> own) {
   Acc3<T> acc{T(0), T(0), T(0), T(0), T(0)};
   bool walls = false;
-  slot_sums<T, W, EXACT, true>(0, i, nc, g, s, own, acc, walls);
+  slot_sums<T, EXACT, true>(0, i, nc, g, s, own, acc, walls);
   if constexpr (EXACT && std::is_same<T, double>::value) {
     // (one copy of the long integer code: unrolled, the stage's instructions
     // no longer stay in the instruction cache)
 #pragma unroll 1
-    for (int k = 1; k < W; ++k) slot_sums<T, W, EXACT, false>(k, i, nc, g, s, own, acc, walls);
+    for (int k = 1; k < W; ++k) slot_sums<T, EXACT, false>(k, i, nc, g, s, own, acc, walls);
   } else {
 #pragma unroll
-    for (int k = 1; k < W; ++k) slot_sums<T, W, EXACT, false>(k, i, nc, g, s, own, acc, walls);
+    for (int k = 1; k < W; ++k) slot_sums<T, EXACT, false>(k, i, nc, g, s, own, acc, walls);
   }
   Vec4<T> d;
   finish<T, EXACT>(acc, walls, __ldg(g.area + i), EXACT ? T(0) : __ldg(g.inv_area + i), d.x, d.y, d.z);

@@ -135,9 +135,9 @@ class CG(esr.Module):
 
     def _fused_solver(self, precision: str):
         """The engine for `precision`: FP64 systems ('native' and 'df64') run
-        on the batched lockstep engine as a batch of one (autotuned work
-        shape, FP64-verified result); 'native' FP32 systems on FusedPCG;
-        'mixed' on MixedPCG."""
+        on the batched engine as a batch of one (FP64-verified result; where
+        the iterations do not run inside one launch, with an autotuned work
+        shape); 'native' FP32 systems on FusedPCG; 'mixed' on MixedPCG."""
         from ..sparse import FusedPCG, MixedPCG, SellMatrix
         A = self.A
 

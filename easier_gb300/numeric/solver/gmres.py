@@ -162,8 +162,9 @@ class GMRES(esr.Module):
               debug_iter: Optional[int] = None, *, fused: Optional[bool] = None) -> Dict[str, Any]:
         """Solve to ``rnorm <= max(rtol*||b||, atol)`` (gmres.py:222-266),
         counting restart cycles.  With a compiled ``Linsys`` and ``M`` None
-        or ``Jacobi`` every restart cycle runs as one CUDA graph of fused
-        kernels (``fused=False`` forces ``gmres_per_op``)."""
+        or ``Jacobi`` the restart cycles run inside cooperative launches of up
+        to 16 cycles, or, for systems too large for one, each as a CUDA graph
+        of fused kernels (``fused=False`` forces ``gmres_per_op``)."""
         name = self.__class__.__name__
 
         def log(it, rn):

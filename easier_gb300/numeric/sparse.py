@@ -247,9 +247,10 @@ GMRES_CYCLES = 16
 
 class FusedGMRES:
     """Restarted GMRES on a SELL matrix with M = Jacobi or identity
-    (gmres.py algorithm): one cooperative launch per restart cycle (or, for
-    systems it does not hold, one CUDA graph of many), one 64-byte read of the
-    device scalars per cycle for the host's stopping test."""
+    (gmres.py algorithm): cooperative launches of up to GMRES_CYCLES restart
+    cycles (or, for systems that do not fit one, a CUDA graph of many launches
+    a cycle), one read of the device scalars a launch or graph for the host's
+    stopping test."""
 
     def __init__(self, A: SellMatrix, restart: int, jacobi: bool = False, use_graph: bool = True):
         self.A = A

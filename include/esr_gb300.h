@@ -608,7 +608,7 @@ int esr_gmres_residual(const esr_sell *A, const void *b, const void *x, void *r,
  * multiprocessors' shared memory (esr_gmres_one_launch; about 3.7 M rows) run
  * it as one cooperative launch with classical Gram-Schmidt applied twice,
  * larger ones as a fixed launch sequence with modified Gram-Schmidt in the
- * reference's order. */
+ * reference's order.  Either can be captured in a CUDA graph. */
 int esr_gmres_one_launch(const esr_sell *A, int32_t restart);
 int esr_gmres_cycle(const esr_sell *A, const void *invdiag, const void *b,
                     void *x, void *r, void *V, void *w2, int32_t restart,
