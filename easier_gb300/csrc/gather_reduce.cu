@@ -371,7 +371,7 @@ int launch_segreduce(int op, const void *t, int64_t cols, const int32_t *rowptr,
 // same rounded operations in the same order (bitwise the five).  One thread
 // a row, four entries' loads in flight, all of x's before the first product
 // (the sum's branches hold loads back); bound in FP64 by latency and the FP64
-// pipe together (two operations an entry, one a row: 75% busy), by HBM in FP32.
+// pipe together (two operations an entry, one a row: 72% busy), by HBM in FP32.
 // 998,001-row P1 grid, FP64: 84 us as five steps; 35 with eight entries and x
 // loaded product by product; 31 so.  The row's own product runs on the integer
 // pipe; the entries' there too: 33.  Two rows a thread: 39.
